@@ -12,8 +12,10 @@
 // (fftcheb_transport.hpp:481-495).
 //
 // B200 layout (the reference's per-row FFTW layout is not kept):
-// * the three right chains are one N x 3R panel ([row][axis][sample]), so a
-//   moment is one wide fused step for them and one narrow one for l;
+// * scalar rows with velocities on H's pattern: all four chains in one panel
+//   and one launch per moment (moment_kernel); otherwise the three right chains
+//   are one N x 3R panel ([row][axis][sample]), so a moment is one wide fused
+//   step for them, one narrow one for l, three current SpMMs and a store copy;
 // * the stores are moment-major, S[m][axis][row][sample], so every moment's
 //   rows land with coalesced writes;
 // * the DCT-III of a chunk of rows is a strided batched inverse 2M-point
@@ -99,6 +101,245 @@ __global__ void store_right_vec_kernel(int64_t row0, int64_t rows, int R, const 
         const int a = int(run / rows);
         dst[e] = src[((row0 + row) * 3 + a) * upr + u];
     }
+}
+
+// ---------------------------------------------------------------------------
+// One moment of both chains in one launch, for scalar rows whose H, Vx, Vy and
+// Vz share a pattern (H real, V_a = i W_a): the route of the orthogonal form
+// of pz operators at a real k-point.
+//
+// The chains live in one panel of 4 W1 reals per row, [row][l, r^x, r^y,
+// r^z][sample], so a nonzero pulls one contiguous run of its neighbour's row,
+// and the four matrices' values sit together ({h, w_x, w_y, w_z} per nonzero,
+// one vector load).  A launch reads moment m (cur) and
+//   writes the currents J_a l_m of the section's rows to the left store,
+//   copies the section's r^a_m to the right store,
+//   replaces moment m - 1 (prev) by moment m + 1 of every row:
+//     y = 2 (Op cur - c cur) / hw - prev   (without the 2 and prev at m = 0),
+// the arithmetic of finish_row (products and sums over the nonzeros in the
+// vectors' precision and in pattern order, rescale and recurrence in FP64), so
+// its results equal those of the separate launches.
+//
+// A thread owns V consecutive reals of one row (16 bytes where the sample
+// count allows, always whole complex values of one chain); C = 4 W1 / V
+// threads share a row.  A CTA's rows are consecutive, so its nonzeros' values
+// and indices are one contiguous run, staged in shared memory: read per thread
+// they were a serial chain of first touches (110 us per moment against 75.8 at
+// 47,632 rows of 33 nonzeros, 16 FP32 samples), and only the gathered rows are
+// left to wait for.  Bound by the latency of those (512 bytes per nonzero, 57 %
+// L1 hits), 32 warps x 4 loads per SM.  The six launches this replaces (left
+// step, right step, three currents, store copy) took 141 us; 11,536 rows x 5
+// FP64 samples: 18.7 us against 51.
+template <typename T>
+struct MomentArgs {
+    int64_t n_rows, row0, row1;  // all rows; the section's rows [row0, row1)
+    const int32_t* row_ptr;
+    const int32_t* col_ind;
+    const T* wgt;                // 4 values per nonzero
+    const T* cur;
+    T* prev;
+    T* sl;                       // this moment's slots of the left and right store
+    T* sr;
+    int W1;                      // reals per row and chain (2 R)
+    int C;                       // threads per row
+    int cap;                     // nonzeros staged per pass
+    int advance;                 // form moment m + 1
+    double c, inv_hw, s2, g_p;   // g_p == 0: no predecessor
+    double cscale;               // -1 / (2 hw)
+};
+
+// Evict-first stores: a moment's store rows are next read by the row stage,
+// after every other moment.
+template <typename T, int V>
+__device__ __forceinline__ void store_stream(T* p, const T (&o)[V]) {
+    if constexpr (sizeof(T) == 8) {
+#pragma unroll
+        for (int i = 0; i < V / 2; ++i)
+            __stcs(reinterpret_cast<double2*>(p) + i, make_double2(o[2 * i], o[2 * i + 1]));
+    } else if constexpr (V % 4 == 0) {
+#pragma unroll
+        for (int i = 0; i < V / 4; ++i)
+            __stcs(reinterpret_cast<float4*>(p) + i,
+                   make_float4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]));
+    } else {
+#pragma unroll
+        for (int i = 0; i < V / 2; ++i)
+            __stcs(reinterpret_cast<float2*>(p) + i, make_float2(o[2 * i], o[2 * i + 1]));
+    }
+}
+
+constexpr int kMomentCap = 640;
+
+template <typename T> struct Vec4;
+template <> struct Vec4<float> {
+    static __device__ __forceinline__ void load(const float* p, float (&w)[4]) {
+        const float4 t = __ldg(reinterpret_cast<const float4*>(p));
+        w[0] = t.x; w[1] = t.y; w[2] = t.z; w[3] = t.w;
+    }
+};
+template <> struct Vec4<double> {
+    static __device__ __forceinline__ void load(const double* p, double (&w)[4]) {
+        const double2 t = __ldg(reinterpret_cast<const double2*>(p));
+        const double2 u = __ldg(reinterpret_cast<const double2*>(p) + 1);
+        w[0] = t.x; w[1] = t.y; w[2] = u.x; w[3] = u.y;
+    }
+};
+
+template <typename T, int V, int U, int MINB>
+__global__ void __launch_bounds__(256, MINB) moment_kernel(MomentArgs<T> a) {
+    extern __shared__ __align__(16) unsigned char msm_raw[];
+    T* sw = reinterpret_cast<T*>(msm_raw);                        // [cap][4]
+    int32_t* sj = reinterpret_cast<int32_t*>(sw + 4 * a.cap);     // [cap]
+    const int C = a.C;
+    const int lr = threadIdx.x / C, ch = threadIdx.x - lr * C;
+    const int64_t i0 = int64_t(blockIdx.x) * (blockDim.x / C);
+    const int64_t i = i0 + lr;
+    const bool live = i < a.n_rows;
+    const bool left = ch < C / 4;
+    const bool in_sec = live && i >= a.row0 && i < a.row1;
+    const bool cur_ax = left && in_sec;  // this thread forms currents
+    const int PW = 4 * a.W1;
+    const T* X = a.cur + ch * V;
+    T acc[V], cx[3][V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) acc[v] = cx[0][v] = cx[1][v] = cx[2][v] = T(0);
+    const int64_t i1 = min(i0 + blockDim.x / C, a.n_rows);
+    const int kb = __ldg(a.row_ptr + i0), ke = __ldg(a.row_ptr + i1);
+    const int k0 = live ? __ldg(a.row_ptr + i) : ke;
+    const int k1 = live ? __ldg(a.row_ptr + i + 1) : ke;
+    // The CTA's nonzeros (consecutive in the pattern) come to shared memory in
+    // passes of cap, coalesced; one pass unless a row is longer than cap.
+    for (int base = kb; base < ke; base += a.cap) {
+        const int m = min(a.cap, ke - base);
+        if (base != kb) __syncthreads();
+        for (int t = threadIdx.x; t < m; t += blockDim.x) {
+            T w[4];
+            Vec4<T>::load(a.wgt + 4 * (int64_t(base) + t), w);
+            sj[t] = __ldg(a.col_ind + base + t);
+            store_vals<T, 4>(sw + 4 * t, w);
+        }
+        __syncthreads();
+        int k = max(k0, base) - base;
+        const int kn = min(k1, base + m) - base;
+        for (; k + U <= kn; k += U) {
+            T x[U][V];
+#pragma unroll
+            for (int u = 0; u < U; ++u) load_vals<T, V>(X + int64_t(sj[k + u]) * PW, x[u]);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const T* w = sw + 4 * (k + u);
+                fma_row<T, V>(acc, w[0], x[u]);
+                if (cur_ax) {
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) fma_row<T, V>(cx[q], w[q + 1], x[u]);
+                }
+            }
+        }
+        if (k < kn) {  // the last, short group: clamped loads, guarded sums
+            T x[U][V];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                load_vals<T, V>(X + int64_t(sj[min(k + u, kn - 1)]) * PW, x[u]);
+#pragma unroll
+            for (int u = 0; u < U - 1; ++u)
+                if (k + u < kn) {
+                    const T* w = sw + 4 * (k + u);
+                    fma_row<T, V>(acc, w[0], x[u]);
+                    if (cur_ax) {
+#pragma unroll
+                        for (int q = 0; q < 3; ++q) fma_row<T, V>(cx[q], w[q + 1], x[u]);
+                    }
+                }
+        }
+    }
+    if (!live) return;
+    T xv[V];
+    load_vals<T, V>(X + i * PW, xv);
+    if (in_sec) {
+        const int64_t rows = a.row1 - a.row0;
+        if (left) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                T o[V];
+#pragma unroll
+                for (int v = 0; v < V; v += 2) {  // i times the real sums
+                    o[v] = T(-double(cx[q][v + 1]) * a.cscale);
+                    o[v + 1] = T(double(cx[q][v]) * a.cscale);
+                }
+                store_stream<T, V>(a.sl + (q * rows + (i - a.row0)) * a.W1 + ch * V, o);
+            }
+        } else {
+            const int q = ch / (C / 4) - 1, e = (ch - (q + 1) * (C / 4)) * V;
+            store_stream<T, V>(a.sr + (q * rows + (i - a.row0)) * a.W1 + e, xv);
+        }
+    }
+    if (!a.advance) return;
+    T* P = a.prev + i * PW + ch * V;
+    T y[V];
+    if (a.g_p != 0.0) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) y[v] = P[v];
+    }
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        double t = fma(-a.c, double(xv[v]), double(acc[v])) * a.inv_hw;
+        if (a.g_p != 0.0) t = fma(a.s2, t, a.g_p * double(y[v]));
+        y[v] = T(t);
+    }
+    store_vals<T, V>(P, y);
+}
+
+// The start of the panel: l_0 = psi, r^a_0 = J_a psi; one thread per (row, sample).
+template <typename T>
+__global__ void moment_init_kernel(int64_t n_rows, int R, const int32_t* row_ptr,
+                                   const int32_t* col_ind, const T* wgt, const T* psi,
+                                   double cscale, T* panel) {
+    const int64_t total = n_rows * R;
+    for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < total;
+         e += int64_t(gridDim.x) * blockDim.x) {
+        const int64_t i = e / R;
+        const int s = int(e - i * R);
+        T cx[3][2] = {{0, 0}, {0, 0}, {0, 0}};
+        for (int k = __ldg(row_ptr + i), k1 = __ldg(row_ptr + i + 1); k < k1; ++k) {
+            T w[4], x[2];
+            load_vals<T, 2>(psi + 2 * (int64_t(__ldg(col_ind + k)) * R + s), x);
+            Vec4<T>::load(wgt + 4 * int64_t(k), w);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) fma_row<T, 2>(cx[q], w[q + 1], x);
+        }
+        T* out = panel + i * 8 * R + 2 * s;
+        out[0] = psi[2 * e];
+        out[1] = psi[2 * e + 1];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            out[2 * (q + 1) * R] = T(-double(cx[q][1]) * cscale);
+            out[2 * (q + 1) * R + 1] = T(double(cx[q][0]) * cscale);
+        }
+    }
+}
+
+// {h, w_x, w_y, w_z} per nonzero; *differs becomes non-zero when a velocity's
+// pattern is not H's (the caller then keeps the separate launches).
+template <typename T>
+__global__ void pack_weights_kernel(int64_t n_rows, int64_t nnz, const int32_t* rp,
+                                    const int32_t* ci, const T* h, const int32_t* rpx,
+                                    const int32_t* cix, const T* wx, const int32_t* rpy,
+                                    const int32_t* ciy, const T* wy, const int32_t* rpz,
+                                    const int32_t* ciz, const T* wz, T* wgt, int* differs) {
+    bool bad = false;
+    for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < nnz;
+         e += int64_t(gridDim.x) * blockDim.x) {
+        const int32_t j = ci[e];
+        bad |= cix[e] != j || ciy[e] != j || ciz[e] != j;
+        const T v[4] = {h[e], wx[e], wy[e], wz[e]};
+        store_vals<T, 4>(wgt + 4 * e, v);
+    }
+    for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e <= n_rows;
+         e += int64_t(gridDim.x) * blockDim.x) {
+        const int32_t r = rp[e];
+        bad |= rpx[e] != r || rpy[e] != r || rpz[e] != r;
+    }
+    if (bad) *differs = 1;
 }
 
 // Even extension with the half-grid phase of fft.hpp:125-154 for a chunk of
@@ -566,6 +807,10 @@ struct DevBuf {
         RSATB_CUDA_TRY(cudaMalloc(&p, bytes));
         return RSATB_SUCCESS;
     }
+    void release() {
+        if (p) cudaFree(p);
+        p = nullptr;
+    }
     template <typename T>
     T* as() const {
         return static_cast<T*>(p);
@@ -668,6 +913,35 @@ unsigned grid_for(int64_t n, int sm) {
     return unsigned(g < 1 ? 1 : g);
 }
 
+// RSATB_FFTCHEB_MOMENT=0: the separate launches of a moment.
+bool moment_enabled() {
+    const char* s = std::getenv("RSATB_FFTCHEB_MOMENT");
+    return !(s && s[0] == '0');
+}
+
+// Threads per row of moment_kernel: 16 bytes each where the samples allow it
+// (FP32: an even sample count; FP64: one complex value).
+template <typename T>
+int moment_threads_per_row(int R) {
+    const int v = sizeof(T) == 4 && R % 2 == 0 ? 4 : 2;
+    return 8 * R / v;
+}
+
+// Orthogonal form, scalar rows, a real H and imaginary-unit velocities with
+// as many nonzeros as H; the patterns themselves are compared on the device.
+bool moment_matrices_ok(const Ctx& c, const rsatb_bsr_matrix* const* V, int R) {
+    const rsatb_bsr_matrix* H = c.op->H;
+    const auto real = [](const rsatb_bsr_matrix* A) { return !dtype_is_complex(A->dtype); };
+    if (c.sandwich || H->block_size != 1 || !real(H) || (H->flags & RSATB_BSR_IMAGINARY_UNIT))
+        return false;
+    if (8 * R / (H->dtype == RSATB_F32 && R % 2 == 0 ? 4 : 2) > 256) return false;
+    for (int a = 0; a < 3; ++a)
+        if (!real(V[a]) || !(V[a]->flags & RSATB_BSR_IMAGINARY_UNIT) ||
+            V[a]->nnz_blocks != H->nnz_blocks)
+            return false;
+    return true;
+}
+
 template <typename T>
 int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, int R, int M,
                  int formulation, double prefactor, int sections, size_t workspace, int kernel,
@@ -684,12 +958,45 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
 
     // Store per block row: both chains, all moments, 3 axes x R samples.
     const size_t store_per_brow = 2 * size_t(M) * b * 3 * R * cplx;
-    const size_t fixed = size_t(N) * cplx * (3 * R /*rinit*/ + 3 * 3 * R /*r*/ + 3 * R /*l*/ +
-                                            3 * R /*J psi*/ + (c.sandwich ? 2 * 3 * R : 0));
+    size_t fixed = size_t(N) * cplx * (3 * R /*rinit*/ + 3 * 3 * R /*r*/ + 3 * R /*l*/ +
+                                      3 * R /*J psi*/ + (c.sandwich ? 2 * 3 * R : 0));
     if (workspace == 0) {
         size_t free_b = 0, total_b = 0;
         RSATB_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
         workspace = free_b / 10 * 8;
+    }
+    // One launch per moment (moment_kernel) where the four matrices allow it
+    // and its buffers (two panels, the start, the packed values) are no larger
+    // than the separate launches' or small in the workspace; RSATB_FFTCHEB_MOMENT=0
+    // keeps the separate launches.
+    DevBuf bPan, bInit, bWgt;
+    const int64_t nnz = c.op->H->nnz_blocks;
+    const size_t fixed_m =
+        size_t(N) * cplx * 3 * 4 * R + 4 * size_t(nnz) * sizeof(T) + sizeof(int) + 256;
+    bool one_launch = moment_enabled() && moment_matrices_ok(c, V, R) &&
+                      fixed_m <= std::max(fixed, workspace / 8);
+    if (one_launch) {
+        RSATB_TRY(bWgt.alloc(4 * size_t(nnz) * sizeof(T) + 256));
+        int* d_differs = reinterpret_cast<int*>(bWgt.as<T>() + 4 * nnz);
+        RSATB_CUDA_TRY(cudaMemsetAsync(d_differs, 0, sizeof(int), st));
+        const rsatb_bsr_matrix* H = c.op->H;
+        pack_weights_kernel<T><<<grid_for(std::max<int64_t>(nnz, N + 1), ctx->sm_count), 256, 0,
+                                 st>>>(
+            N, nnz, H->row_ptr, H->col_ind, static_cast<const T*>(H->values), V[0]->row_ptr,
+            V[0]->col_ind, static_cast<const T*>(V[0]->values), V[1]->row_ptr, V[1]->col_ind,
+            static_cast<const T*>(V[1]->values), V[2]->row_ptr, V[2]->col_ind,
+            static_cast<const T*>(V[2]->values), bWgt.as<T>(), d_differs);
+        RSATB_LAUNCH_CHECK(ctx);
+        int differs = 0;
+        RSATB_CUDA_TRY(cudaMemcpyAsync(&differs, d_differs, sizeof(int), cudaMemcpyDeviceToHost,
+                                       st));
+        RSATB_CUDA_TRY(cudaStreamSynchronize(st));
+        if (differs) {
+            one_launch = false;
+            bWgt.release();
+        } else {
+            fixed = fixed_m;
+        }
     }
     if (workspace <= fixed + store_per_brow)
         return set_error(RSATB_OUT_OF_MEMORY,
@@ -724,10 +1031,16 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
 
     // Buffers.
     DevBuf bJ, bRinit, bR, bL, bU, bW, bS, bE, bK, bWts;
-    RSATB_TRY(bJ.alloc(size_t(N) * 3 * R * cplx));
-    RSATB_TRY(bRinit.alloc(size_t(N) * 3 * R * cplx));
-    RSATB_TRY(bR.alloc(size_t(N) * 3 * 3 * R * cplx));
-    RSATB_TRY(bL.alloc(size_t(N) * 3 * R * cplx));
+    const size_t panel = size_t(N) * 8 * R;  // reals of one moment_kernel panel
+    if (one_launch) {
+        RSATB_TRY(bPan.alloc(2 * panel * sizeof(T)));
+        RSATB_TRY(bInit.alloc(panel * sizeof(T)));
+    } else {
+        RSATB_TRY(bJ.alloc(size_t(N) * 3 * R * cplx));
+        RSATB_TRY(bRinit.alloc(size_t(N) * 3 * R * cplx));
+        RSATB_TRY(bR.alloc(size_t(N) * 3 * 3 * R * cplx));
+        RSATB_TRY(bL.alloc(size_t(N) * 3 * R * cplx));
+    }
     if (c.sandwich) {
         RSATB_TRY(bU.alloc(size_t(N) * 3 * R * cplx));
         RSATB_TRY(bW.alloc(size_t(N) * 3 * R * cplx));
@@ -851,11 +1164,37 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
     float rec_ms = 0.f, dct_ms = 0.f;
 
     // J_a psi and the right-chain start.
-    for (int a = 0; a < 3; ++a)
-        RSATB_TRY(current_rows(c, V[a], W1, psi, J[a], 0, nb, bU.p, bW.p));
-    pack_axes_kernel<T><<<grid_for(N * 3 * R, ctx->sm_count), 256, 0, st>>>(N, R, J[0], J[1],
-                                                                           J[2], rinit);
-    RSATB_LAUNCH_CHECK(ctx);
+    MomentArgs<T> ma{};
+    int m_threads = 0;
+    size_t m_smem = 0;
+    if (one_launch) {
+        ma.n_rows = N;
+        ma.row_ptr = c.op->H->row_ptr;
+        ma.col_ind = c.op->H->col_ind;
+        ma.wgt = bWgt.as<T>();
+        ma.W1 = W1;
+        ma.C = moment_threads_per_row<T>(R);
+        ma.c = c.op->center;
+        ma.inv_hw = 1.0 / c.op->half_width;
+        ma.cscale = -1.0 / (2.0 * c.op->half_width);
+        // Rows per CTA: up to 256 threads, and as many as fit one pass of
+        // kMomentCap nonzeros.
+        const int longest = std::max(1, c.op->H->max_row_blocks);
+        int rpc = std::min(256 / ma.C, kMomentCap / longest);
+        if (rpc < 1) rpc = 1;
+        m_threads = rpc * ma.C;
+        ma.cap = std::min(kMomentCap, rpc * longest);
+        m_smem = size_t(ma.cap) * (4 * sizeof(T) + sizeof(int32_t));
+        moment_init_kernel<T><<<grid_for(N * R, ctx->sm_count), 256, 0, st>>>(
+            N, R, ma.row_ptr, ma.col_ind, ma.wgt, psi, ma.cscale, bInit.as<T>());
+        RSATB_LAUNCH_CHECK(ctx);
+    } else {
+        for (int a = 0; a < 3; ++a)
+            RSATB_TRY(current_rows(c, V[a], W1, psi, J[a], 0, nb, bU.p, bW.p));
+        pack_axes_kernel<T><<<grid_for(N * 3 * R, ctx->sm_count), 256, 0, st>>>(N, R, J[0], J[1],
+                                                                               J[2], rinit);
+        RSATB_LAUNCH_CHECK(ctx);
+    }
 
     int64_t chunks = 0;
     for (int sec = 0; sec < n_sections; ++sec) {
@@ -865,52 +1204,87 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
         const int64_t rows = int64_t(sb1 - sb0) * b;
         const int64_t sslot = 3 * rows * R;  // this section's slot size
         RSATB_CUDA_TRY(cudaEventRecord(ev0, st));
-        RSATB_CUDA_TRY(cudaMemcpyAsync(r[0], rinit, size_t(N) * 3 * R * cplx,
-                                       cudaMemcpyDeviceToDevice, st));
-        const T* lp = psi;       // l_{m-1}
-        const T* lc = nullptr;   // l_m
-        int ri_prev = 0, ri_cur = -1;
-        int li = 0;
-        for (int m = 0; m < M; ++m) {
-            const T* lm;  // l_m
-            int rm;       // index of r_m
-            if (m == 0) {
-                lm = psi;
-                rm = 0;
-            } else if (m == 1) {
-                T* lo = l[li];
-                li = (li + 1) % 3;
-                RSATB_TRY(op_step(c, W1, lp, nullptr, lo, bU.p, bW.p, 1.0, 0.0));
-                RSATB_TRY(op_step(c, W3, r[ri_prev], nullptr, r[1], bU.p, bW.p, 1.0, 0.0));
-                lc = lo;
-                ri_cur = 1;
-                lm = lc;
-                rm = 1;
-            } else {
-                T* lo = l[li];
-                li = (li + 1) % 3;
-                const int rn = 3 - ri_prev - ri_cur;
-                RSATB_TRY(op_step(c, W1, lc, lp, lo, bU.p, bW.p, 2.0, -1.0));
-                RSATB_TRY(op_step(c, W3, r[ri_cur], r[ri_prev], r[rn], bU.p, bW.p, 2.0, -1.0));
-                lp = lc;
-                lc = lo;
-                ri_prev = ri_cur;
-                ri_cur = rn;
-                lm = lc;
-                rm = rn;
+        if (one_launch) {
+            // Moment 0 is read from its own buffer, moment 1 formed in panel 0,
+            // then the panels alternate (panel 1 takes moment 2 over a copy of
+            // moment 0, its predecessor).
+            T* pan[2] = {bPan.as<T>(), bPan.as<T>() + panel};
+            if (M > 1)
+                RSATB_CUDA_TRY(cudaMemcpyAsync(pan[1], bInit.p, panel * sizeof(T),
+                                               cudaMemcpyDeviceToDevice, st));
+            const int rpc = m_threads / ma.C;
+            const unsigned grid = unsigned((N + rpc - 1) / rpc);
+            ma.row0 = rows0;
+            ma.row1 = rows0 + rows;
+            for (int m = 0; m < M; ++m) {
+                ma.cur = m == 0 ? bInit.as<T>() : pan[(m + 1) & 1];
+                ma.prev = pan[m & 1];
+                ma.sl = SL + 2 * size_t(m) * sslot;
+                ma.sr = SR + 2 * size_t(m) * sslot;
+                ma.advance = m + 1 < M;
+                ma.s2 = m == 0 ? 1.0 : 2.0;
+                ma.g_p = m == 0 ? 0.0 : -1.0;
+                // Resident CTAs against loads in flight (us per moment, 47,632
+                // rows, 16 FP32 samples): 4 CTAs x 4 loads 75.8, 3 x 4 86.9,
+                // 3 x 8 84.2, 5 x 2 90.0.
+                if constexpr (sizeof(T) == 4) {
+                    if (R % 2 == 0)
+                        moment_kernel<T, 4, 4, 4><<<grid, m_threads, m_smem, st>>>(ma);
+                    else
+                        moment_kernel<T, 2, 4, 5><<<grid, m_threads, m_smem, st>>>(ma);
+                } else {
+                    moment_kernel<T, 2, 4, 4><<<grid, m_threads, m_smem, st>>>(ma);
+                }
+                RSATB_LAUNCH_CHECK(ctx);
             }
-            T* sl = SL + 2 * size_t(m) * sslot;
-            for (int a = 0; a < 3; ++a)
-                RSATB_TRY(current_rows(c, V[a], W1, lm, sl + 2 * size_t(a) * rows * R, sb0, sb1,
-                                       bU.p, bW.p));
-            if (sizeof(T) == 8 || R % 2 == 0)
-                store_right_vec_kernel<T>
-                    <<<grid_for(sslot * 2 * int64_t(sizeof(T)) / 16, ctx->sm_count), 256, 0, st>>>(
+        } else {
+            RSATB_CUDA_TRY(cudaMemcpyAsync(r[0], rinit, size_t(N) * 3 * R * cplx,
+                                           cudaMemcpyDeviceToDevice, st));
+            const T* lp = psi;       // l_{m-1}
+            const T* lc = nullptr;   // l_m
+            int ri_prev = 0, ri_cur = -1;
+            int li = 0;
+            for (int m = 0; m < M; ++m) {
+                const T* lm;  // l_m
+                int rm;       // index of r_m
+                if (m == 0) {
+                    lm = psi;
+                    rm = 0;
+                } else if (m == 1) {
+                    T* lo = l[li];
+                    li = (li + 1) % 3;
+                    RSATB_TRY(op_step(c, W1, lp, nullptr, lo, bU.p, bW.p, 1.0, 0.0));
+                    RSATB_TRY(op_step(c, W3, r[ri_prev], nullptr, r[1], bU.p, bW.p, 1.0, 0.0));
+                    lc = lo;
+                    ri_cur = 1;
+                    lm = lc;
+                    rm = 1;
+                } else {
+                    T* lo = l[li];
+                    li = (li + 1) % 3;
+                    const int rn = 3 - ri_prev - ri_cur;
+                    RSATB_TRY(op_step(c, W1, lc, lp, lo, bU.p, bW.p, 2.0, -1.0));
+                    RSATB_TRY(op_step(c, W3, r[ri_cur], r[ri_prev], r[rn], bU.p, bW.p, 2.0, -1.0));
+                    lp = lc;
+                    lc = lo;
+                    ri_prev = ri_cur;
+                    ri_cur = rn;
+                    lm = lc;
+                    rm = rn;
+                }
+                T* sl = SL + 2 * size_t(m) * sslot;
+                for (int a = 0; a < 3; ++a)
+                    RSATB_TRY(current_rows(c, V[a], W1, lm, sl + 2 * size_t(a) * rows * R, sb0, sb1,
+                                           bU.p, bW.p));
+                if (sizeof(T) == 8 || R % 2 == 0)
+                    store_right_vec_kernel<T>
+                        <<<grid_for(sslot * 2 * int64_t(sizeof(T)) / 16, ctx->sm_count), 256, 0, st>>>(
+                            rows0, rows, R, r[rm], SR + 2 * size_t(m) * sslot);
+                else
+                    store_right_kernel<T><<<grid_for(sslot, ctx->sm_count), 256, 0, st>>>(
                         rows0, rows, R, r[rm], SR + 2 * size_t(m) * sslot);
-            else
-                store_right_kernel<T><<<grid_for(sslot, ctx->sm_count), 256, 0, st>>>(
-                    rows0, rows, R, r[rm], SR + 2 * size_t(m) * sslot);
-            RSATB_LAUNCH_CHECK(ctx);
+                RSATB_LAUNCH_CHECK(ctx);
+            }
         }
         RSATB_CUDA_TRY(cudaEventRecord(ev1, st));
         RSATB_CUDA_TRY(cudaEventSynchronize(ev1));

@@ -302,3 +302,72 @@ def test_fused_row_stage_at_2048_moments(torch_cuda, precision, monkeypatch):
         sig_o, en_o = _oracle(H, V, psi, 2048, emin, emax)
         assert np.allclose(en, en_o, rtol=0, atol=1e-13)
         assert rel_err(fused, sig_o) < 1e-10
+
+
+def _scalar_chain(n, long_row, seed):
+    """A real symmetric scalar-row H on a ring with one row of long_row
+    nonzeros, and real antisymmetric W_a on the same pattern."""
+    from rsatb_b200 import lattice
+    rng = np.random.default_rng(seed)
+    A = np.zeros((n, n), dtype=bool)
+    i = np.arange(n)
+    A[i, (i + 1) % n] = A[i, i] = True
+    A[3, rng.permutation(n)[:long_row]] = True
+    A |= A.T
+    h = np.triu(rng.standard_normal((n, n)))
+    h = (h + np.triu(h, 1).T) / np.sqrt(max(3, long_row))
+    rp = np.concatenate([[0], np.cumsum(A.sum(1))]).astype(np.int32)
+    ci = np.nonzero(A)[1].astype(np.int32)
+    bsr = lambda v: lattice.BsrArrays(rp, ci, v[A].reshape(-1, 1, 1), 1)  # noqa: E731
+    V = []
+    for _ in range(3):
+        w = np.triu(rng.standard_normal((n, n)), 1)
+        V.append(bsr(w - w.T))
+    return bsr(h), V
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+@pytest.mark.parametrize("n,long_row,R,M,kw", [
+    (5, 0, 1, 1, {}),                             # one moment, fewer rows than a CTA
+    (301, 0, 1, 2, {}),
+    (301, 0, 3, 17, {"partition_sections": 4}),   # rows outside the section
+    (900, 700, 2, 9, {}),                         # a row longer than one staging pass
+    (900, 899, 5, 8, {"partition_sections": 2}),
+    (130, 40, 16, 12, {"formulation": 1}),
+    (130, 40, 64, 6, {}),                         # the widest FP64 row of one CTA
+    (130, 40, 65, 6, {}),                         # beyond it: the separate launches
+])
+def test_one_launch_per_moment_equals_the_separate_launches(torch_cuda, monkeypatch, precision, n,
+                                                            long_row, R, M, kw):
+    """Same products in the same order: equal to the last bit of the rounding of
+    the sums after them."""
+    H, V = _scalar_chain(n, long_row, seed=n + R)
+    psi = _phases(n, R, seed=2)
+    args = (torch_cuda, H, V, psi, M, -8.0, 8.0, precision)
+    one = _gpu(*args, **kw)[0]
+    monkeypatch.setenv("RSATB_FFTCHEB_MOMENT", "0")
+    six = _gpu(*args, **kw)[0]
+    assert np.abs(six).max() > 0 or M < 2
+    assert rel_err(one, six) <= (1e-13 if precision == "f64" else 1e-6)
+
+
+def test_velocity_of_another_pattern_keeps_the_separate_launches(torch_cuda):
+    """Vy with as many nonzeros as H in other places: against the oracle."""
+    from rsatb_b200 import lattice
+    H, V = _scalar_chain(40, 0, seed=8)
+    order = np.argsort(H.col_ind[H.row_ptr[0]:H.row_ptr[1]])
+    assert order.size == 3
+    n = 40
+    W = np.zeros((n, n))
+    i = np.arange(n)
+    W[i, (i + 2) % n] = 0.7
+    W = W - W.T
+    mask = W != 0
+    mask[i, i] = True  # a stored zero diagonal: three entries per row, as H
+    rp = np.concatenate([[0], np.cumsum(mask.sum(1))]).astype(np.int32)
+    ci = np.nonzero(mask)[1].astype(np.int32)
+    V[1] = lattice.BsrArrays(rp, ci, W[mask].reshape(-1, 1, 1), 1)
+    assert V[1].nnz_blocks == H.nnz_blocks
+    psi = _phases(n, 3, seed=6)
+    sig = _gpu(torch_cuda, H, V, psi, 24, -8.0, 8.0)[0]
+    assert rel_err(sig, _oracle(H, V, psi, 24, -8.0, 8.0)[0]) < 1e-10
