@@ -71,26 +71,26 @@ extern "C" int rsatb_evaluate_kpm_density(rsatb_ctx_t ctx, const double* moments
         return RSATB_SUCCESS;
     }
     // g_n * Re(mu_n) on the host: n_moments products, as kpm.hpp forms them.
-    std::vector<double> g(n_moments), gmu(n_moments);
+    // With x behind them, one copy into the context's scratch (stream-ordered
+    // allocations here went back to the device at every synchronisation and
+    // cost 0.45 ms a call).
+    std::vector<double> g(n_moments), in(size_t(n_moments) + nx);
     kpm_kernel_weights(kernel, n_moments, g.data());
-    for (int n = 0; n < n_moments; ++n) gmu[n] = g[n] * moments[2 * n];
-    double *d_gmu = nullptr, *d_x = nullptr, *d_rho = nullptr;
-    RSATB_CUDA_TRY(cudaMallocAsync(&d_gmu, sizeof(double) * n_moments, ctx->stream));
-    RSATB_CUDA_TRY(cudaMallocAsync(&d_x, sizeof(double) * nx, ctx->stream));
-    RSATB_CUDA_TRY(cudaMallocAsync(&d_rho, sizeof(double) * nx, ctx->stream));
-    RSATB_CUDA_TRY(cudaMemcpyAsync(d_gmu, gmu.data(), sizeof(double) * n_moments,
+    for (int n = 0; n < n_moments; ++n) in[n] = g[n] * moments[2 * n];
+    std::copy(x, x + nx, in.begin() + n_moments);
+    void* s = nullptr;
+    RSATB_TRY(ctx_scratch(ctx, sizeof(double) * (in.size() + nx), &s));
+    double* d_gmu = static_cast<double*>(s);
+    double* d_x = d_gmu + n_moments;
+    double* d_rho = d_x + nx;
+    RSATB_CUDA_TRY(cudaMemcpyAsync(d_gmu, in.data(), sizeof(double) * in.size(),
                                    cudaMemcpyHostToDevice, ctx->stream));
-    RSATB_CUDA_TRY(cudaMemcpyAsync(d_x, x, sizeof(double) * nx, cudaMemcpyHostToDevice,
-                                   ctx->stream));
     const int threads = 128;
     kpm_density_kernel<<<(nx + threads - 1) / threads, threads, 0, ctx->stream>>>(
         d_gmu, n_moments, d_x, nx, edge_inset, d_rho);
     RSATB_LAUNCH_CHECK(ctx);
     RSATB_CUDA_TRY(cudaMemcpyAsync(rho_out, d_rho, sizeof(double) * nx, cudaMemcpyDeviceToHost,
                                    ctx->stream));
-    cudaFreeAsync(d_gmu, ctx->stream);
-    cudaFreeAsync(d_x, ctx->stream);
-    cudaFreeAsync(d_rho, ctx->stream);
     RSATB_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     return RSATB_SUCCESS;
 }
