@@ -51,6 +51,11 @@ struct StepArgs {
     double* dots_out;  // [ndots][W]
     unsigned* counter;
     unsigned* fault;   // set non-zero by a kernel whose bounded wait gave up (null: none)
+    void* ax;          // optional sum over the recurrence, ax += (ax_re + i ax_im) y, by the
+                       // kernels that take it (step_takes_ax); null: none
+    double ax_re, ax_im;
+    int ax_init;       // ax starts here as (ax0_re + i ax0_im) x instead of its contents
+    double ax0_re, ax0_im;
     int wait_check;    // non-zero: the bulk-copy kernel only runs a wait that cannot
                        // complete (a 5 ms limit), to check the fault report
 };
@@ -141,10 +146,35 @@ __device__ __forceinline__ void fma_row(VT (&acc)[V], VT a, const VT (&x)[V]) {
     }
 }
 
+// ax += c y for V values of one row, rounded as the separate launch rounds
+// (the start c0 x too); a real panel takes Re(c).
+template <typename VT, int V, bool CV>
+__device__ __forceinline__ void add_ax(const StepArgs& a, int64_t off, const VT (&xv)[V],
+                                       const VT (&yv)[V]) {
+    VT* o = static_cast<VT*>(a.ax) + off;
+    VT s[V];
+    const auto mul = [](double re, double im, const VT (&z)[V], int v) {
+        if constexpr (CV)
+            return v & 1 ? re * double(z[v]) + im * double(z[v - 1])
+                         : re * double(z[v]) - im * double(z[v + 1]);
+        else
+            return re * double(z[v]);
+    };
+    if (a.ax_init) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) s[v] = VT(mul(a.ax0_re, a.ax0_im, xv, v));
+    } else {
+        load_vals<VT, V, true>(o, s);
+    }
+#pragma unroll
+    for (int v = 0; v < V; ++v) s[v] = VT(double(s[v]) + mul(a.ax_re, a.ax_im, yv, v));
+    store_vals<VT, V>(o, s);
+}
+
 // Epilogue for one output row: rescale, recurrence, store, dots.  CG: the
 // x, p, q and psi0 panels are read through L2 (written earlier in the same
 // launch).
-template <typename VT, int V, bool CV, bool CG = false>
+template <typename VT, int V, bool CV, bool CG = false, bool AX = false>
 __device__ __forceinline__ void finish_row(const StepArgs& a, int64_t row, int g,
                                            const VT (&acc)[V], double (&d0)[V],
                                            double (&d1)[V]) {
@@ -193,6 +223,9 @@ __device__ __forceinline__ void finish_row(const StepArgs& a, int64_t row, int g
 #pragma unroll
     for (int v = 0; v < V; ++v) yv[v] = VT(t[v]);
     store_vals<VT, V>(static_cast<VT*>(a.y) + off, yv);
+    if constexpr (AX) {
+        if (a.ax) add_ax<VT, V, CV>(a, off, xv, yv);
+    }
 
     if (a.dot_mode == DOT_DOUBLING) {
         // <y|x> and <y|y>, from the stored (rounded) y.
@@ -380,10 +413,16 @@ __global__ void __launch_bounds__(256) cheb_step_kernel(StepArgs a) {
         }
 #pragma unroll
         for (int r = 0; r < B; ++r)
-            finish_row<VT, V, CV>(a, i * B + r, g, acc[r], d0, d1);
+            finish_row<VT, V, CV, false, B == 1>(a, i * B + r, g, acc[r], d0, d1);
     }
     if (a.dot_mode != DOT_NONE) reduce_dots<V>(a, L, d0, d1);
 }
+
+// Whether a step on A adds into StepArgs::ax: the register kernel of scalar
+// rows does (its default), where the separate launch that reads the step's
+// output back was a third of a term (graphene, 80,000 rows x 4 FP64 complex
+// columns: 5.7 + 3.2 us in two launches, 7.6 in one).
+bool step_takes_ax(const rsatb_bsr_matrix* A);
 
 // Runtime block size (b <= 16): the fallback for block sizes without a
 // specialisation.  Same arithmetic, rows of the block handled one at a time.

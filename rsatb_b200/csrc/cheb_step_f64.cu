@@ -8,6 +8,10 @@ int launch_cheb_step_f64(rsatb_context* ctx, const rsatb_bsr_matrix* A, int vec_
     return step_detail::launch_step_precision<double>(ctx, A, vec_dtype, args);
 }
 
+bool step_takes_ax(const rsatb_bsr_matrix* A) {
+    return A->block_size == 1 && step_detail::env_kernel() == 0;
+}
+
 int launch_coldot_f64(rsatb_context* ctx, int vec_dtype, int64_t n_rows, StepArgs args) {
     return step_detail::launch_coldot_precision<double>(ctx, vec_dtype, n_rows, args);
 }

@@ -637,10 +637,14 @@ int rsatb_cheb_propagate(rsatb_ctx_t ctx, const rsatb_cheb_op* op, const void* X
     void* buf[3] = {base, base + vbytes, base + 2 * vbytes};
     void* u = sh.sandwich ? base + 3 * vbytes : nullptr;
     void* w = sh.sandwich ? base + 4 * vbytes : nullptr;
+    // Scalar rows add every term in the step's epilogue.
+    const bool in_step = n_coeffs > 1 && !sh.sandwich && step_takes_ax(op->H);
     // Y = c_0 T_0 X = c_0 X (cheby.hpp:399-441): zero, then add.
-    RSATB_CUDA_TRY(cudaMemsetAsync(Y, 0, size_t(n_values) * dtype_real_size(vec_dtype),
-                                   ctx->stream));
-    RSATB_TRY(axpy_coeff(ctx, vec_dtype, n_values, coeffs[0], coeffs[1], X, Y));
+    if (!in_step) {
+        RSATB_CUDA_TRY(cudaMemsetAsync(Y, 0, size_t(n_values) * dtype_real_size(vec_dtype),
+                                       ctx->stream));
+        RSATB_TRY(axpy_coeff(ctx, vec_dtype, n_values, coeffs[0], coeffs[1], X, Y));
+    }
     const double inv_hw = 1.0 / op->half_width;
     const void* prev = nullptr;  // T_{n-2} X
     const void* cur = X;         // T_{n-1} X
@@ -649,6 +653,26 @@ int rsatb_cheb_propagate(rsatb_ctx_t ctx, const rsatb_cheb_op* op, const void* X
         void* out = buf[slot];
         slot = (slot + 1) % 3;
         // T_1 = Op~ X; T_n = 2 Op~ T_{n-1} - T_{n-2}
+        if (in_step) {
+            StepArgs a = blank_args(W);
+            a.in = a.x = cur;
+            a.p = n == 1 ? nullptr : prev;
+            a.y = out;
+            a.c = op->center;
+            a.s_out = inv_hw;
+            a.s2 = n == 1 ? 1.0 : 2.0;
+            a.g_p = n == 1 ? 0.0 : -1.0;
+            a.ax = Y;
+            a.ax_re = coeffs[2 * n];
+            a.ax_im = coeffs[2 * n + 1];
+            a.ax_init = n == 1;
+            a.ax0_re = coeffs[0];
+            a.ax0_im = coeffs[1];
+            RSATB_TRY(run_step(ctx, op->H, vec_dtype, a));
+            prev = cur;
+            cur = out;
+            continue;
+        }
         RSATB_TRY(apply_fused(ctx, op, sh, vec_dtype, W, cur, cur, n == 1 ? nullptr : prev, out, u,
                               w, inv_hw, n == 1 ? 1.0 : 2.0, n == 1 ? 0.0 : -1.0, DOT_NONE,
                               nullptr, nullptr, nullptr, nullptr));
