@@ -25,8 +25,9 @@
 // backward pass holds O(sqrt(N)) panels, not N.  Each backward step is one
 // fused step kernel (the a_n psi term rides in its epilogue); each segment
 // ends with one SDDMM launch over the C moments of the segment.
-#include "cheb_kernels.cuh"
+#include "cheb_dmma.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -94,10 +95,123 @@ __global__ void __launch_bounds__(256) sddmm_kernel(int n_block_rows, const int3
     }
 }
 
+// The same sampled products on the FP64 tensor cores, blocks of 4 to 8: the
+// sum over (moment, sample) is the contraction index k' = q R + s of
+// mma.sync m8n8k4 tiles (rows r, columns c of the block, zero lanes beyond b).
+// A warp takes kSdBlocks consecutive blocks of one block row: L_i's fragment is
+// loaded once for all of them and there is no reduction at the end (the tile
+// is the block).  Lane fc takes k' = 8 t + 2 fc and + 1 for two tiles of a step
+// (the order of a sum's terms is free), one 2-value load each when R is even.
+// Bound by the loads of T_j in flight from L2; 69,632 blocks of 5, 32 FP64
+// samples, a segment of 16 moments: 261 us against 891 a warp per (block, row).
+constexpr int kSdBlocks = 6;
+
+template <typename VT, bool PAIR>
+__global__ void __launch_bounds__(128) sddmm_dmma_kernel(int n_block_rows, int n_chunks, int b,
+                                                         const int32_t* row_ptr,
+                                                         const int32_t* col_ind, int R, int n0,
+                                                         int len, double scale, const VT* L,
+                                                         const VT* T, int64_t panel,
+                                                         double* grad) {
+    const int lane = threadIdx.x & 31;
+    const int fr = lane >> 2, fc = lane & 3;
+    const int row = min(fr, b - 1);  // rows and columns beyond b are dropped
+    const int64_t items = int64_t(n_block_rows) * n_chunks;
+    const int K = len * R;
+    const int dq = 8 / R, ds = 8 - dq * R;
+    for (int64_t it = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); it < items;
+         it += int64_t(gridDim.x) * (blockDim.x >> 5)) {
+        const int64_t i = it / n_chunks;
+        const int kb = __ldg(row_ptr + i) + int(it - i * n_chunks) * kSdBlocks;
+        const int ke = min(__ldg(row_ptr + i + 1), kb + kSdBlocks);
+        if (kb >= ke) continue;
+        const VT* Lr = L + (i * b + row) * R;
+        const VT* Tr[kSdBlocks];
+#pragma unroll
+        for (int u = 0; u < kSdBlocks; ++u)
+            Tr[u] = T + (int64_t(__ldg(col_ind + min(kb + u, ke - 1))) * b + row) * R;
+        double acc[kSdBlocks][2];
+#pragma unroll
+        for (int u = 0; u < kSdBlocks; ++u) acc[u][0] = acc[u][1] = 0.0;
+        // (q, s) of this lane's two k'
+        int q0 = 2 * fc / R, s0 = 2 * fc - q0 * R;
+        int q1 = (2 * fc + 1) / R, s1 = 2 * fc + 1 - q1 * R;
+        for (int t = 2 * fc; t - 2 * fc < K; t += 8) {
+            const bool v0 = t < K, v1 = t + 1 < K;
+            const int64_t o0 = v0 ? q0 * panel + s0 : 0, o1 = v1 ? q1 * panel + s1 : 0;
+            VT l0, l1, t0[kSdBlocks], t1[kSdBlocks];
+            const auto pair = [&](const VT* p, VT& x, VT& y) {
+                if constexpr (PAIR && sizeof(VT) == 8) {
+                    const double2 w = __ldg(reinterpret_cast<const double2*>(p + o0));
+                    x = w.x;
+                    y = w.y;
+                } else if constexpr (PAIR) {
+                    const float2 w = __ldg(reinterpret_cast<const float2*>(p + o0));
+                    x = w.x;
+                    y = w.y;
+                } else {
+                    x = __ldg(p + o0);
+                    y = __ldg(p + o1);
+                }
+            };
+            pair(Lr, l0, l1);
+#pragma unroll
+            for (int u = 0; u < kSdBlocks; ++u) pair(Tr[u], t0[u], t1[u]);
+            const double a0 = v0 ? (n0 + q0 ? 2.0 : 1.0) * double(l0) : 0.0;
+            const double a1 = v1 ? (n0 + q1 ? 2.0 : 1.0) * double(l1) : 0.0;
+#pragma unroll
+            for (int u = 0; u < kSdBlocks; ++u) {
+                dmma_884(acc[u], a0, v0 ? double(t0[u]) : 0.0);
+                dmma_884(acc[u], a1, v1 ? double(t1[u]) : 0.0);
+            }
+            q0 += dq;
+            s0 += ds;
+            if (s0 >= R) {
+                s0 -= R;
+                ++q0;
+            }
+            q1 += dq;
+            s1 += ds;
+            if (s1 >= R) {
+                s1 -= R;
+                ++q1;
+            }
+        }
+        if (fr < b) {
+#pragma unroll
+            for (int u = 0; u < kSdBlocks; ++u)
+                if (kb + u < ke) {
+                    double* g = grad + (int64_t(kb + u) * b + fr) * b;
+#pragma unroll
+                    for (int v = 0; v < 2; ++v)
+                        if (2 * fc + v < b) g[2 * fc + v] += scale * acc[u][v];
+                }
+        }
+    }
+}
+
 template <typename VT>
 int launch_sddmm(rsatb_context* ctx, const rsatb_bsr_matrix* H, int R, int n0, int len,
                  int n_last, double scale, const VT* L, const VT* T, int64_t panel,
                  double* grad) {
+    // Blocks of 4 to 8 fill the 8 x 8 tiles from a quarter up; below that the
+    // warp-per-row kernel does no zero work.
+    const int used = std::min(len, n_last - n0 + 1);
+    if (H->block_size >= 4 && H->block_size <= 8) {
+        if (used <= 0 || H->nnz_blocks == 0) return RSATB_SUCCESS;
+        const int chunks = (std::max(1, H->max_row_blocks) + kSdBlocks - 1) / kSdBlocks;
+        int64_t g = (int64_t(H->n_block_rows) * chunks + 3) / 4;
+        if (g > int64_t(ctx->sm_count) * 32) g = int64_t(ctx->sm_count) * 32;
+        const bool pair = R % 2 == 0 && panel % 2 == 0 &&
+                          ((reinterpret_cast<uintptr_t>(L) | reinterpret_cast<uintptr_t>(T)) &
+                           (2 * sizeof(VT) - 1)) == 0;
+        auto kern = pair ? sddmm_dmma_kernel<VT, true> : sddmm_dmma_kernel<VT, false>;
+        kern<<<unsigned(g), 128, 0, ctx->stream>>>(H->n_block_rows, chunks, H->block_size,
+                                                   H->row_ptr, H->col_ind, R, n0, used, scale, L,
+                                                   T, panel, grad);
+        RSATB_LAUNCH_CHECK(ctx);
+        return RSATB_SUCCESS;
+    }
     const int64_t items = H->nnz_blocks * H->block_size;
     int64_t grid = (items + 7) / 8;
     if (grid > int64_t(ctx->sm_count) * 16) grid = int64_t(ctx->sm_count) * 16;
@@ -109,9 +223,6 @@ int launch_sddmm(rsatb_context* ctx, const rsatb_bsr_matrix* H, int R, int n0, i
         case 1: RSATB_SDDMM(1); break;
         case 2: RSATB_SDDMM(2); break;
         case 3: RSATB_SDDMM(3); break;
-        case 4: RSATB_SDDMM(4); break;
-        case 5: RSATB_SDDMM(5); break;
-        case 8: RSATB_SDDMM(8); break;
         default:
             return set_error(RSATB_NOT_SUPPORTED, "gradient for block size %d not built",
                              H->block_size);
@@ -289,17 +400,24 @@ int vjp_impl(rsatb_context* ctx, const rsatb_cheb_op* op, const VT* psi, int R, 
                 RSATB_TRY(step(cur, prv, out, 2.0, -1.0, nullptr, 0.0, nullptr));
             }
         }
+        // lambda_{n+1} pairs with t_n in the gradient: slot n of the segment.
+        // With C >= 3 lambda_n is formed in its slot n - 1 (its predecessors sit
+        // two and three slots above, or, at the segment's top, in lam and in the
+        // slots 0 and 1 that this segment writes last); only the lambda carried
+        // into a segment is copied.  Shorter segments copy every one.
         for (int n = nb1 - 1; n >= nb0; --n) {
-            // lambda_{n+1} pairs with t_n in the gradient
-            RSATB_CUDA_TRY(cudaMemcpyAsync(lseg + size_t(n - nb0) * ps, l1, pbytes,
-                                           cudaMemcpyDeviceToDevice, st));
+            VT* slot = lseg + size_t(n - nb0) * ps;
+            if (l1 != slot)
+                RSATB_CUDA_TRY(cudaMemcpyAsync(slot, l1, pbytes, cudaMemcpyDeviceToDevice, st));
             if (n >= 1) {
-                VT* out = lam + size_t(ls) * ps;
-                while (out == l1 || out == l2) {
+                VT* out = C >= 3 && n > nb0 ? slot - ps : lam + size_t(ls) * ps;
+                if (C < 3 || n == nb0) {
+                    while (out == l1 || out == l2) {
+                        ls = (ls + 1) % 3;
+                        out = lam + size_t(ls) * ps;
+                    }
                     ls = (ls + 1) % 3;
-                    out = lam + size_t(ls) * ps;
                 }
-                ls = (ls + 1) % 3;
                 RSATB_TRY(step(l1, l2, out, 2.0, -1.0, psi, dmu[n] / double(R), nullptr));
                 l2 = l1;
                 l1 = out;
