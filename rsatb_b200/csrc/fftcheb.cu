@@ -18,9 +18,9 @@
 //   step for them, one narrow one for l, three current SpMMs and a store copy;
 // * the stores are moment-major, S[m][axis][row][sample], so every moment's
 //   rows land with coalesced writes;
-// * the DCT-III of a chunk of rows is a strided batched inverse 2M-point
-//   FFT (cuFFT, sequences interleaved: stride = batch) of the half-grid
-//   phased even extension, built and read back with coalesced accesses;
+// * the DCT-III of a chunk of rows is a strided batched inverse M-point
+//   FFT (cuFFT, sequences interleaved: stride = batch) of dct3_input_kernel's
+//   sequences, built and read back with coalesced accesses;
 // * the contraction gives each energy k to one CTA per chunk: no atomics,
 //   the same summation order on every run;
 // * at M = 2048 (Greenwood) the row stage is one hand-written kernel after a
@@ -342,32 +342,50 @@ __global__ void pack_weights_kernel(int64_t n_rows, int64_t nnz, const int32_t* 
     if (bad) *differs = 1;
 }
 
-// Even extension with the half-grid phase of fft.hpp:125-154 for a chunk of
-// sequences: sequence q (0 <= q < nq, q = (a * chunk_rows + row) * R + s,
-// rows offset row_off inside the section) of store S (slot stride
-// slot_elems complex entries, section rows sec_rows) weighted by w_m:
-//   E[0][q] = w_0 x_0,   E[m][q] = w_m x_m e^{i pi m / 2M},
-//   E[2M - m][q] = w_m x_m e^{-i pi m / 2M}  (1 <= m < M),   E[M][q] = 0.
+// Input of the M-point transform that gives the DCT-III of fft.hpp:125-154
+//   y_k = w_0 x_0 + 2 sum_{m >= 1} w_m x_m cos(pi m (k + 1/2) / M)
+// for a chunk of sequences: sequence q (0 <= q < nq, q = (a * chunk_rows + row)
+// * R + s, rows offset row_off inside the section) of store S (slot stride
+// slot_elems complex entries, section rows sec_rows) weighted by w_m.
+//   F_0 = w_0 x_0,  F_m = e^{i pi m / 2M} (w_m x_m - i w_{M-m} x_{M-m}),
+// whose inverse DFT v_p = sum_m F_m e^{2 pi i m p / M} holds y in the order of
+// dct3_energy (Makhoul, IEEE Trans. ASSP 28, 27, 1980; linear in x, so complex
+// x is two real transforms at once): half the points and half the buffer of
+// the even extension's 2M-point transform.  One thread reads x_m and x_{M-m}
+// and writes F_m and F_{M-m}; blockIdx.y is m <= M / 2.
+__host__ __device__ inline int dct3_energy(int M, int p) {
+    return p < (M + 1) / 2 ? 2 * p : 2 * (M - 1 - p) + 1;
+}
+
 template <typename T>
-__global__ void extend_kernel(int M, int64_t nq, int chunk_rows, int R, int64_t sec_rows,
-                              int64_t row_off, int64_t slot_elems, const T* S, const double* w,
-                              double2* E) {
-    const int m = blockIdx.y;
-    const double th = M_PI * double(m) / (2.0 * double(M));
-    const double c = cos(th), sn = sin(th);
+__global__ void dct3_input_kernel(int M, int64_t nq, int chunk_rows, int R, int64_t sec_rows,
+                                  int64_t row_off, int64_t slot_elems, const T* S,
+                                  const double* w, double2* F) {
+    const int m = blockIdx.y, mm = M - m;
+    double c, sn;
+    sincospi(double(m) / (2.0 * double(M)), &sn, &c);
+    const double wm = w[m], wr = m ? w[mm] : 0.0;
     for (int64_t q = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; q < nq;
          q += int64_t(gridDim.x) * blockDim.x) {
         const int s = int(q % R);
         const int64_t row = (q / R) % chunk_rows;
         const int a = int(q / (int64_t(chunk_rows) * R));
-        const int64_t src = int64_t(m) * slot_elems + (a * sec_rows + row_off + row) * R + s;
-        const double xr = w[m] * double(S[2 * src]), xi = w[m] * double(S[2 * src + 1]);
+        const int64_t src = (a * sec_rows + row_off + row) * R + s;
+        const T* p = S + 2 * (int64_t(m) * slot_elems + src);
+        const double xr = wm * double(p[0]), xi = wm * double(p[1]);
         if (m == 0) {
-            E[q] = make_double2(xr, xi);
-            E[int64_t(M) * nq + q] = make_double2(0.0, 0.0);
-        } else {
-            E[int64_t(m) * nq + q] = make_double2(xr * c - xi * sn, xr * sn + xi * c);
-            E[int64_t(2 * M - m) * nq + q] = make_double2(xr * c + xi * sn, -xr * sn + xi * c);
+            F[q] = make_double2(xr, xi);
+            continue;
+        }
+        const T* pr = S + 2 * (int64_t(mm) * slot_elems + src);
+        const double zr = wr * double(pr[0]), zi = wr * double(pr[1]);
+        // x - i z, times (c + i sn)
+        const double ar = xr + zi, ai = xi - zr;
+        F[int64_t(m) * nq + q] = make_double2(ar * c - ai * sn, ar * sn + ai * c);
+        if (mm != m) {
+            // z - i x, times e^{i pi (M - m) / 2M} = sn + i c
+            const double br = zr + xi, bi = zi - xr;
+            F[int64_t(mm) * nq + q] = make_double2(br * sn - bi * c, br * c + bi * sn);
         }
     }
 }
@@ -393,14 +411,16 @@ __global__ void pad_kernel(int M, int64_t nq, int chunk_rows, int R, int64_t sec
     }
 }
 
-// Bastin kernel accumulation (fftcheb_transport.hpp:496-519): for energy k
+// Bastin kernel accumulation (fftcheb_transport.hpp:496-519), phi3 (the DCT-III)
+// taken from phi1's transform: its angles are theta_k = pi (k + 1/2) / M and
+// theta_{2M-1-k} = 2 pi - theta_k, so phi3_k = (phi1_k + phi1_{2M-1-k}) / 2.
+// For energy k
 // (one CTA) and every component (a, b), a <= b,
 //   K[k][ab] += sum over rows, samples of
 //     eps_k (conj(L3_a) R1_b + conj(L1_a) R3_b)
 //     + i sqrt(1 - eps_k^2) (conj(L2_a) R3_b - conj(L3_a) R2_b),
 // summed per thread, then in a fixed tree order (deterministic).
 __global__ void __launch_bounds__(256) bastin_contract_kernel(int M, int64_t nq, int64_t per_axis,
-                                                              const double2* L3, const double2* R3,
                                                               const double2* L1, const double2* R1,
                                                               const double2* L2, const double2* R2,
                                                               double* K) {
@@ -409,7 +429,10 @@ __global__ void __launch_bounds__(256) bastin_contract_kernel(int M, int64_t nq,
     const double eps = cos(th), root = sin(th);
     __shared__ double red[12][256];
     double acc[6][2] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}};
-    const int64_t o = int64_t(k) * nq;
+    const int64_t o = int64_t(k) * nq, o2 = int64_t(2 * M - 1 - k) * nq;
+    const auto half_sum = [](double2 x, double2 y) {
+        return make_double2(0.5 * (x.x + y.x), 0.5 * (x.y + y.y));
+    };
     // conj(x) y, accumulated into (re, im)
     auto cmac = [](double (&d)[2], double2 x, double2 y, double f_re, double f_im) {
         const double re = x.x * y.x + x.y * y.y, im = x.x * y.y - x.y * y.x;
@@ -420,12 +443,12 @@ __global__ void __launch_bounds__(256) bastin_contract_kernel(int M, int64_t nq,
         int comp = 0;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            const double2 l3 = L3[o + a * per_axis + q], l1 = L1[o + a * per_axis + q],
-                          l2 = L2[o + a * per_axis + q];
+            const double2 l1 = L1[o + a * per_axis + q], l2 = L2[o + a * per_axis + q];
+            const double2 l3 = half_sum(l1, L1[o2 + a * per_axis + q]);
 #pragma unroll
             for (int b = a; b < 3; ++b, ++comp) {
-                const double2 r3 = R3[o + b * per_axis + q], r1 = R1[o + b * per_axis + q],
-                              r2 = R2[o + b * per_axis + q];
+                const double2 r1 = R1[o + b * per_axis + q], r2 = R2[o + b * per_axis + q];
+                const double2 r3 = half_sum(r1, R1[o2 + b * per_axis + q]);
                 cmac(acc[comp], l3, r1, eps, 0.0);
                 cmac(acc[comp], l1, r3, eps, 0.0);
                 cmac(acc[comp], l2, r3, 0.0, root);
@@ -448,20 +471,21 @@ __global__ void __launch_bounds__(256) bastin_contract_kernel(int M, int64_t nq,
 }
 
 // K[k][a] += sum over the chunk's (row, s) of conj(L3[k][q]) R3[k][q] /
-// max(1e-14, 1 - eps_k^2): one CTA per energy k, fixed order.
+// max(1e-14, 1 - eps_k^2): one CTA per transform output p (energy
+// dct3_energy(M, p)), fixed order.
 __global__ void __launch_bounds__(256) greenwood_contract_kernel(int M, int64_t nq,
                                                                  int64_t per_axis,
                                                                  const double2* L3,
                                                                  const double2* R3,
                                                                  double* K) {
-    const int k = blockIdx.x;
+    const int k = dct3_energy(M, blockIdx.x);
     const double eps = cos(M_PI * (double(k) + 0.5) / double(M));
     const double wden = 1.0 - eps * eps;
     const double inv = 1.0 / (wden > 1e-14 ? wden : 1e-14);
     __shared__ double red[3][2][256];
     double acc[3][2] = {{0, 0}, {0, 0}, {0, 0}};
-    const double2* l = L3 + int64_t(k) * nq;
-    const double2* r = R3 + int64_t(k) * nq;
+    const double2* l = L3 + int64_t(blockIdx.x) * nq;
+    const double2* r = R3 + int64_t(blockIdx.x) * nq;
     for (int a = 0; a < 3; ++a)
         for (int64_t q = threadIdx.x; q < per_axis; q += blockDim.x) {
             const double2 x = l[a * per_axis + q], y = r[a * per_axis + q];
@@ -947,7 +971,9 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
                  int formulation, double prefactor, int sections, size_t workspace, int kernel,
                  double* sigma_out, double* energy_out, rsatb_fftcheb_stats* stats) {
     const bool bastin = formulation == 1;
-    const int n_tf = bastin ? 3 : 1;  // transforms per side and row: phi3 (+ phi1, phi2)
+    // Transform points per side and sequence: the M-point DCT-III, or Bastin's
+    // zero-padded 2M-point phi1 and phi2 (phi3 comes out of phi1).
+    const int n_pts = bastin ? 4 * M : M;
     rsatb_context* ctx = c.ctx;
     cudaStream_t st = ctx->stream;
     const int b = c.op->H->block_size;
@@ -1014,7 +1040,7 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
         fused ? std::max(2 * size_t(M) * cplx, std::min(avail / 4, fused_chunk_bytes))
               : avail / 4;
     const size_t fft_per_row =
-        size_t(n_tf) * 2 * 2 * size_t(M) * 3 * R * sizeof(double2) * 2;  // + cuFFT work
+        2 * size_t(n_pts) * 3 * R * sizeof(double2) * 2;  // + cuFFT work
     int64_t chunk_rows = int64_t(fft_budget / fft_per_row);
     if (chunk_rows < 1) chunk_rows = 1;
     int64_t sec_brows = int64_t((avail - fft_budget) / store_per_brow);
@@ -1050,7 +1076,7 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
     RSATB_TRY(bS.alloc(2 * size_t(M) * slot * cplx));
     const int64_t nq_max = 3 * chunk_rows * R;
     const size_t e_bytes =
-        fused ? fft_budget : size_t(n_tf) * 2 * 2 * size_t(M) * nq_max * sizeof(double2);
+        fused ? fft_budget : 2 * size_t(n_pts) * nq_max * sizeof(double2);
     RSATB_TRY(bE.alloc(e_bytes));
     RSATB_TRY(bK.alloc(size_t(M) * 12 * sizeof(double)));
     RSATB_TRY(bWts.alloc(size_t(M) * sizeof(double)));
@@ -1068,12 +1094,12 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
     T* SL = bS.as<T>();
     T* SR = SL + 2 * size_t(M) * slot;
     double2* EL = bE.as<double2>();
-    double2* ER = fused ? nullptr : EL + 2 * size_t(M) * nq_max;
-    // Bastin: phi1 and phi2 of both sides follow.
-    double2* EL1 = bastin ? ER + 2 * size_t(M) * nq_max : nullptr;
-    double2* ER1 = bastin ? EL1 + 2 * size_t(M) * nq_max : nullptr;
-    double2* EL2 = bastin ? ER1 + 2 * size_t(M) * nq_max : nullptr;
-    double2* ER2 = bastin ? EL2 + 2 * size_t(M) * nq_max : nullptr;
+    double2* ER = EL + size_t(M) * nq_max;
+    // Bastin: phi1 and phi2 of both sides.
+    double2* EL1 = EL;
+    double2* ER1 = EL1 + 2 * size_t(M) * nq_max;
+    double2* EL2 = ER1 + 2 * size_t(M) * nq_max;
+    double2* ER2 = EL2 + 2 * size_t(M) * nq_max;
     double* K = bK.as<double>();
 
     std::vector<double> g(M), wts(M);
@@ -1140,8 +1166,8 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
             cufftDestroy(plans[slot_i].h);
             plans[slot_i].made = false;
         }
-        int n2 = 2 * M;
-        int emb = 2 * M;
+        int n2 = bastin ? 2 * M : M;
+        int emb = n2;
         RSATB_CUFFT_TRY(cufftPlanMany(&plans[slot_i].h, 1, &n2, &emb, int(nq), 1, &emb, int(nq), 1,
                                       CUFFT_Z2Z, int(nq)));
         plans[slot_i].made = true;
@@ -1333,23 +1359,24 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
             const int64_t nq = 3 * cr * R;
             cufftHandle plan;
             RSATB_TRY(plan_for(nq, &plan));
-            dim3 grid(grid_for(nq, ctx->sm_count) > 64 ? 64 : grid_for(nq, ctx->sm_count), M);
-            extend_kernel<T><<<grid, 256, 0, st>>>(M, nq, int(cr), R, rows, c0, sslot, SL,
-                                                   bWts.as<double>(), EL);
-            RSATB_LAUNCH_CHECK(ctx);
-            extend_kernel<T><<<grid, 256, 0, st>>>(M, nq, int(cr), R, rows, c0, sslot, SR,
-                                                   bWts.as<double>(), ER);
-            RSATB_LAUNCH_CHECK(ctx);
-            RSATB_CUFFT_TRY(cufftExecZ2Z(plan, reinterpret_cast<cufftDoubleComplex*>(EL),
-                                         reinterpret_cast<cufftDoubleComplex*>(EL),
-                                         CUFFT_INVERSE));
-            RSATB_CUFFT_TRY(cufftExecZ2Z(plan, reinterpret_cast<cufftDoubleComplex*>(ER),
-                                         reinterpret_cast<cufftDoubleComplex*>(ER),
-                                         CUFFT_INVERSE));
+            const unsigned gx = std::min(64u, grid_for(nq, ctx->sm_count));
             if (!bastin) {
+                const dim3 grid(gx, M / 2 + 1);
+                const T* src[2] = {SL, SR};
+                double2* dst[2] = {EL, ER};
+                for (int t = 0; t < 2; ++t) {
+                    dct3_input_kernel<T><<<grid, 256, 0, st>>>(M, nq, int(cr), R, rows, c0, sslot,
+                                                               src[t], bWts.as<double>(), dst[t]);
+                    RSATB_LAUNCH_CHECK(ctx);
+                    RSATB_CUFFT_TRY(cufftExecZ2Z(plan,
+                                                 reinterpret_cast<cufftDoubleComplex*>(dst[t]),
+                                                 reinterpret_cast<cufftDoubleComplex*>(dst[t]),
+                                                 CUFFT_INVERSE));
+                }
                 greenwood_contract_kernel<<<M, 256, 0, st>>>(M, nq, cr * R, EL, ER, K);
                 RSATB_LAUNCH_CHECK(ctx);
             } else {
+                const dim3 grid(gx, M);
                 const double2* w1 = bPw.as<double2>();
                 const double2* w2 = w1 + M;
                 double2* dst[4] = {EL1, ER1, EL2, ER2};
@@ -1363,8 +1390,7 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
                                                  reinterpret_cast<cufftDoubleComplex*>(dst[t]),
                                                  CUFFT_INVERSE));
                 }
-                bastin_contract_kernel<<<M, 256, 0, st>>>(M, nq, cr * R, EL, ER, EL1, ER1, EL2,
-                                                          ER2, K);
+                bastin_contract_kernel<<<M, 256, 0, st>>>(M, nq, cr * R, EL1, ER1, EL2, ER2, K);
                 RSATB_LAUNCH_CHECK(ctx);
             }
             ++chunks;
