@@ -173,11 +173,15 @@ __device__ __forceinline__ void add_ax(const StepArgs& a, int64_t off, const VT 
 
 // Epilogue for one output row: rescale, recurrence, store, dots.  CG: the
 // x, p, q and psi0 panels are read through L2 (written earlier in the same
-// launch).
+// launch).  px, pp, pq, p0: the x, p, q and psi0 values where the caller has read
+// them already (so that their latency runs beside other work: the branches here
+// keep the loads of one row's groups from overlapping).
 template <typename VT, int V, bool CV, bool CG = false, bool AX = false>
 __device__ __forceinline__ void finish_row(const StepArgs& a, int64_t row, int g,
                                            const VT (&acc)[V], double (&d0)[V],
-                                           double (&d1)[V]) {
+                                           double (&d1)[V], const VT* px = nullptr,
+                                           const VT* pp = nullptr, const VT* pq = nullptr,
+                                           const VT* p0 = nullptr) {
     const int64_t off = row * a.W + int64_t(g) * V;
     double t[V];
 #pragma unroll
@@ -192,7 +196,10 @@ __device__ __forceinline__ void finish_row(const StepArgs& a, int64_t row, int g
         }
     }
     VT xv[V];
-    if (a.x) {
+    if (px) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) xv[v] = px[v];
+    } else if (a.x) {
         load_vals<VT, V, CG>(static_cast<const VT*>(a.x) + off, xv);
     } else {
 #pragma unroll
@@ -206,7 +213,12 @@ __device__ __forceinline__ void finish_row(const StepArgs& a, int64_t row, int g
     }
     if (a.p) {
         VT pv[V];
-        load_vals<VT, V, CG>(static_cast<const VT*>(a.p) + off, pv);
+        if (pp) {
+#pragma unroll
+            for (int v = 0; v < V; ++v) pv[v] = pp[v];
+        } else {
+            load_vals<VT, V, CG>(static_cast<const VT*>(a.p) + off, pv);
+        }
 #pragma unroll
         for (int v = 0; v < V; ++v) t[v] = fma(a.s2, t[v], a.g_p * double(pv[v]));
     } else if (a.s2 != 1.0) {
@@ -215,7 +227,12 @@ __device__ __forceinline__ void finish_row(const StepArgs& a, int64_t row, int g
     }
     if (a.q) {
         VT qv[V];
-        load_vals<VT, V, CG>(static_cast<const VT*>(a.q) + off, qv);
+        if (pq) {
+#pragma unroll
+            for (int v = 0; v < V; ++v) qv[v] = pq[v];
+        } else {
+            load_vals<VT, V, CG>(static_cast<const VT*>(a.q) + off, qv);
+        }
 #pragma unroll
         for (int v = 0; v < V; ++v) t[v] = fma(a.g_q, double(qv[v]), t[v]);
     }
@@ -248,7 +265,12 @@ __device__ __forceinline__ void finish_row(const StepArgs& a, int64_t row, int g
         }
     } else if (a.dot_mode == DOT_PLAIN) {
         VT qv[V];
-        load_vals<VT, V, CG>(static_cast<const VT*>(a.psi0) + off, qv);
+        if (p0) {
+#pragma unroll
+            for (int v = 0; v < V; ++v) qv[v] = p0[v];
+        } else {
+            load_vals<VT, V, CG>(static_cast<const VT*>(a.psi0) + off, qv);
+        }
         if constexpr (CV) {
 #pragma unroll
             for (int v = 0; v < V; v += 2) {
@@ -264,67 +286,87 @@ __device__ __forceinline__ void finish_row(const StepArgs& a, int64_t row, int g
     }
 }
 
-// After every CTA wrote its partial dots: the last CTA to arrive (ticket
-// counter) sums the gridDim.x partials of each of the O = ndots * W outputs
-// and resets the counter for the next launch.  With fewer outputs than
-// threads, T = blockDim / O threads share an output (CTAs b = part, part + T,
-// ...) and their sums are combined in part order; otherwise each thread takes
-// whole outputs with eight independent accumulators, so the L2 loads of one
-// output are in flight together.  The order is fixed for a given grid:
-// deterministic dots.  Needs blockDim.x <= 256.
-// CTAs of at most 256 threads (comb below), which every step kernel uses.
-__device__ __forceinline__ void finish_partials(const StepArgs& a, int ndots) {
-    __threadfence();
-    __syncthreads();
-    __shared__ unsigned ticket;
+// dst[o] = sum of n partial vectors of O values at P, P + step, ... (elements):
+// T = blockDim / O threads share an output where there are more threads than
+// outputs, their sums combined in part order; otherwise each thread takes whole
+// outputs.  Sixteen loads in flight per thread; a fixed order.  dst may be the
+// first vector.  All the CTA's threads (at most 256) call it.
+__device__ __forceinline__ void sum_partials(const double* P, int n, size_t step, int O,
+                                             double* dst) {
     __shared__ double comb[256];
-    if (threadIdx.x == 0) ticket = atomicAdd(a.counter, 1u);
-    __syncthreads();
-    if (ticket != gridDim.x - 1) return;
-    __threadfence();
-    const int O = ndots * a.W;
     const int nt = blockDim.x;
-    const unsigned G = gridDim.x;
-    const double* P = a.partials;
-    if (O * 2 > nt) {
-        for (int idx = threadIdx.x; idx < O; idx += nt) {
-            double s0 = 0, s1 = 0, s2 = 0, s3 = 0, s4 = 0, s5 = 0, s6 = 0, s7 = 0;
-            unsigned b = 0;
-            for (; b + 8 <= G; b += 8) {
-                s0 += __ldcg(P + size_t(b) * O + idx);
-                s1 += __ldcg(P + size_t(b + 1) * O + idx);
-                s2 += __ldcg(P + size_t(b + 2) * O + idx);
-                s3 += __ldcg(P + size_t(b + 3) * O + idx);
-                s4 += __ldcg(P + size_t(b + 4) * O + idx);
-                s5 += __ldcg(P + size_t(b + 5) * O + idx);
-                s6 += __ldcg(P + size_t(b + 6) * O + idx);
-                s7 += __ldcg(P + size_t(b + 7) * O + idx);
+    const int T = max(1, nt / O);  // threads per output
+    const int part = T > 1 ? threadIdx.x / O : 0;
+    for (int o = T > 1 ? threadIdx.x % O : threadIdx.x; o < O; o += T > 1 ? O : nt) {
+        double sum = 0.0;
+        if (part < T)
+            for (int b = part; b < n; b += 16 * T) {
+                double v[16];
+#pragma unroll
+                for (int u = 0; u < 16; ++u)
+                    v[u] = b + u * T < n ? __ldcg(P + size_t(b + u * T) * step + o) : 0.0;
+#pragma unroll
+                for (int h = 8; h > 0; h >>= 1)
+#pragma unroll
+                    for (int u = 0; u < h; ++u) v[u] += v[u + h];
+                sum += v[0];
             }
-            for (; b < G; ++b) s0 += __ldcg(P + size_t(b) * O + idx);
-            a.dots_out[idx] = ((s0 + s1) + (s2 + s3)) + ((s4 + s5) + (s6 + s7));
-        }
-    } else {
-        const int T = nt / O;
-        const int o = threadIdx.x % O, part = threadIdx.x / O;
-        double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-        if (part < T) {
-            unsigned b = part;
-            for (; b + 3 * T < G; b += 4 * T) {
-                s0 += __ldcg(P + size_t(b) * O + o);
-                s1 += __ldcg(P + size_t(b + T) * O + o);
-                s2 += __ldcg(P + size_t(b + 2 * T) * O + o);
-                s3 += __ldcg(P + size_t(b + 3 * T) * O + o);
-            }
-            for (; b < G; b += T) s0 += __ldcg(P + size_t(b) * O + o);
-        }
-        comb[threadIdx.x] = (s0 + s1) + (s2 + s3);
+        if (T > 1)
+            comb[threadIdx.x] = sum;
+        else
+            dst[o] = sum;
+    }
+    if (T > 1) {
         __syncthreads();
         if (threadIdx.x < O) {
             double t = 0.0;
             for (int q = 0; q < T; ++q) t += comb[q * O + threadIdx.x];
-            a.dots_out[threadIdx.x] = t;
+            dst[threadIdx.x] = t;
         }
     }
+}
+
+// After every CTA wrote its partial dots: the last CTA to arrive (ticket
+// counters) sums them over the CTAs.  In two levels above 32 CTAs: the last of
+// every 32 sums its group's partials in place of the group's first, the last of
+// those sums the groups.  The sums sit on the step's critical path as a chain of
+// L2 round trips: at 1,024 CTAs of 24 outputs the step takes 34 us with one level
+// and four loads in flight, 30 with sixteen, 24 with both levels (17 without
+// dots); FP64 blocks of 8 at W = 32 58.9 -> 47.7, W = 16 38.0 -> 30.0.  The order is fixed for a given grid: deterministic dots.  Resets the
+// counters for the next launch.  Needs blockDim.x <= 256.
+constexpr int kGroupCtas = 32;
+constexpr int kGroupCounter0 = 8;   // the groups' counters: counter[8 + group]
+constexpr int kMaxGroups = 48;      // the fault word lies beyond them
+__device__ __forceinline__ void finish_partials(const StepArgs& a, int ndots) {
+    __threadfence();
+    __syncthreads();
+    __shared__ unsigned ticket;
+    const int O = ndots * a.W;
+    const int G = int(gridDim.x);
+    int n = G;
+    size_t step = O;
+    const int groups = (G + kGroupCtas - 1) / kGroupCtas;
+    if (groups > 1 && groups <= kMaxGroups) {
+        const int group = blockIdx.x / kGroupCtas;
+        const int size = min(kGroupCtas, G - group * kGroupCtas);
+        unsigned* gc = a.counter + kGroupCounter0 + group;
+        if (threadIdx.x == 0) ticket = atomicAdd(gc, 1u);
+        __syncthreads();
+        if (ticket != unsigned(size - 1)) return;
+        __threadfence();
+        if (threadIdx.x == 0) *gc = 0u;
+        double* P = a.partials + size_t(group) * kGroupCtas * O;
+        sum_partials(P, size, O, O, P);
+        n = groups;
+        step = size_t(kGroupCtas) * O;
+        __threadfence();
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) ticket = atomicAdd(a.counter, 1u);
+    __syncthreads();
+    if (ticket != unsigned(n - 1)) return;
+    __threadfence();
+    sum_partials(a.partials, n, step, O, a.dots_out);
     if (threadIdx.x == 0) *a.counter = 0u;  // ready for the next launch
 }
 
@@ -380,6 +422,49 @@ __global__ void __launch_bounds__(256) cheb_step_kernel(StepArgs a) {
 #pragma unroll
             for (int v = 0; v < V; ++v) acc[r][v] = VT(0);
         const int k0 = __ldg(a.row_ptr + i), k1 = __ldg(a.row_ptr + i + 1);
+        if constexpr (B == 1 && !CM) {
+            // Scalar rows: x and p first, then four nonzeros in flight.
+            const int64_t off = i * a.W + int64_t(g) * V;
+            VT xv[V], pv[V];
+#pragma unroll
+            for (int v = 0; v < V; ++v) xv[v] = pv[v] = VT(0);
+            if (a.x) load_vals<VT, V>(static_cast<const VT*>(a.x) + off, xv);
+            if (a.p) load_vals<VT, V>(static_cast<const VT*>(a.p) + off, pv);
+            const VT* X = in + int64_t(g) * V;
+            int k = k0;
+            for (; k + 4 <= k1; k += 4) {
+                int j[4];
+                MT w[4];
+                VT xb[4][V];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    j[u] = __ldg(a.col_ind + k + u);
+                    w[u] = __ldg(vals + k + u);
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) load_vals<VT, V>(X + int64_t(j[u]) * a.W, xb[u]);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) fma_row<VT, V>(acc[0], VT(w[u]), xb[u]);
+            }
+            if (k < k1) {  // one to three left: clamped loads, guarded sums
+                int j[3];
+                MT w[3];
+                VT xb[3][V];
+#pragma unroll
+                for (int u = 0; u < 3; ++u) {
+                    const int kc = min(k + u, k1 - 1);
+                    j[u] = __ldg(a.col_ind + kc);
+                    w[u] = __ldg(vals + kc);
+                }
+#pragma unroll
+                for (int u = 0; u < 3; ++u) load_vals<VT, V>(X + int64_t(j[u]) * a.W, xb[u]);
+#pragma unroll
+                for (int u = 0; u < 3; ++u)
+                    if (k + u < k1) fma_row<VT, V>(acc[0], VT(w[u]), xb[u]);
+            }
+            finish_row<VT, V, CV, false, true>(a, i, g, acc[0], d0, d1, xv, pv);
+            continue;
+        }
         for (int k = k0; k < k1; ++k) {
             const int64_t j = __ldg(a.col_ind + k);
             // X_j: B rows x V values of this thread's columns.

@@ -159,10 +159,11 @@ extern "C" int rsatb_kpm_dos_moments_noalloc(rsatb_ctx_t ctx, const rsatb_cheb_o
                          need, kNoAllocScratchBytes);
     unsigned char* base = nullptr;
     RSATB_TRY(scratch_address(ctx->device, &base));
-    // Header: the dot reductions' completion counter at byte 0, the step
-    // kernels' fault word at byte 128.
+    // Header: the dot reductions' completion counter at byte 0 and their group
+    // counters behind it (kGroupCounter0), the step kernels' fault word at byte
+    // 248.
     unsigned* counter = reinterpret_cast<unsigned*>(base);
-    unsigned* fault = reinterpret_cast<unsigned*>(base + 128);
+    unsigned* fault = reinterpret_cast<unsigned*>(base + 248);
     unsigned char* p = base + 256;
     void* buf[3] = {p, p + vbytes, p + 2 * vbytes};
     void* u = sandwich ? p + 3 * vbytes : nullptr;
