@@ -97,14 +97,16 @@ __global__ void __launch_bounds__(256) sddmm_kernel(int n_block_rows, const int3
 
 // The same sampled products on the FP64 tensor cores, blocks of 4 to 8: the
 // sum over (moment, sample) is the contraction index k' = q R + s of
-// mma.sync m8n8k4 tiles (rows r, columns c of the block, zero lanes beyond b).
-// A warp takes kSdBlocks consecutive blocks of one block row: L_i's fragment is
-// loaded once for all of them and there is no reduction at the end (the tile
-// is the block).  Lane fc takes k' = 8 t + 2 fc and + 1 for two tiles of a step
-// (the order of a sum's terms is free), one 2-value load each when R is even.
-// Bound by the loads of T_j in flight from L2; 69,632 blocks of 5, 32 FP64
-// samples, a segment of 16 moments: 261 us against 891 a warp per (block, row).
-constexpr int kSdBlocks = 6;
+// mma.sync m8n8k4 tiles.  The tile rows are the block's rows (dropped beyond b),
+// the tile columns run over the columns of all the block row's blocks, so blocks
+// of 5 waste none; a warp takes kSdTiles tiles of one block row, L_i's fragment
+// loaded once for all of them, and there is no reduction at the end.  Lane fc
+// takes k' = 8 t + 2 fc and + 1 for the two tiles of a step (the order of a sum's
+// terms is free), one 2-value load each when R is even.
+// Bound by the FP64 tensor pipe; 69,632 blocks of 5, 32 FP64 samples, a segment
+// of 16 moments: 213 us (261 with a tile per block, 891 with a warp per
+// (block, row) and a shuffle tree).
+constexpr int kSdTiles = 6;
 
 template <typename VT, bool PAIR>
 __global__ void __launch_bounds__(128) sddmm_dmma_kernel(int n_block_rows, int n_chunks, int b,
@@ -115,31 +117,34 @@ __global__ void __launch_bounds__(128) sddmm_dmma_kernel(int n_block_rows, int n
                                                          double* grad) {
     const int lane = threadIdx.x & 31;
     const int fr = lane >> 2, fc = lane & 3;
-    const int row = min(fr, b - 1);  // rows and columns beyond b are dropped
+    const int row = min(fr, b - 1);  // rows beyond b are dropped
     const int64_t items = int64_t(n_block_rows) * n_chunks;
     const int K = len * R;
     const int dq = 8 / R, ds = 8 - dq * R;
     for (int64_t it = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); it < items;
          it += int64_t(gridDim.x) * (blockDim.x >> 5)) {
         const int64_t i = it / n_chunks;
-        const int kb = __ldg(row_ptr + i) + int(it - i * n_chunks) * kSdBlocks;
-        const int ke = min(__ldg(row_ptr + i + 1), kb + kSdBlocks);
-        if (kb >= ke) continue;
+        const int kb = __ldg(row_ptr + i);
+        const int cols = (__ldg(row_ptr + i + 1) - kb) * b;  // of the whole block row
+        const int col0 = int(it - i * n_chunks) * 8 * kSdTiles;
+        if (col0 >= cols) continue;
         const VT* Lr = L + (i * b + row) * R;
-        const VT* Tr[kSdBlocks];
+        const VT* Tr[kSdTiles];
 #pragma unroll
-        for (int u = 0; u < kSdBlocks; ++u)
-            Tr[u] = T + (int64_t(__ldg(col_ind + min(kb + u, ke - 1))) * b + row) * R;
-        double acc[kSdBlocks][2];
+        for (int u = 0; u < kSdTiles; ++u) {
+            const int n = min(col0 + 8 * u + fr, cols - 1), blk = n / b;
+            Tr[u] = T + (int64_t(__ldg(col_ind + kb + blk)) * b + (n - blk * b)) * R;
+        }
+        double acc[kSdTiles][2];
 #pragma unroll
-        for (int u = 0; u < kSdBlocks; ++u) acc[u][0] = acc[u][1] = 0.0;
+        for (int u = 0; u < kSdTiles; ++u) acc[u][0] = acc[u][1] = 0.0;
         // (q, s) of this lane's two k'
         int q0 = 2 * fc / R, s0 = 2 * fc - q0 * R;
         int q1 = (2 * fc + 1) / R, s1 = 2 * fc + 1 - q1 * R;
         for (int t = 2 * fc; t - 2 * fc < K; t += 8) {
             const bool v0 = t < K, v1 = t + 1 < K;
             const int64_t o0 = v0 ? q0 * panel + s0 : 0, o1 = v1 ? q1 * panel + s1 : 0;
-            VT l0, l1, t0[kSdBlocks], t1[kSdBlocks];
+            VT l0, l1, t0[kSdTiles], t1[kSdTiles];
             const auto pair = [&](const VT* p, VT& x, VT& y) {
                 if constexpr (PAIR && sizeof(VT) == 8) {
                     const double2 w = __ldg(reinterpret_cast<const double2*>(p + o0));
@@ -156,11 +161,11 @@ __global__ void __launch_bounds__(128) sddmm_dmma_kernel(int n_block_rows, int n
             };
             pair(Lr, l0, l1);
 #pragma unroll
-            for (int u = 0; u < kSdBlocks; ++u) pair(Tr[u], t0[u], t1[u]);
+            for (int u = 0; u < kSdTiles; ++u) pair(Tr[u], t0[u], t1[u]);
             const double a0 = v0 ? (n0 + q0 ? 2.0 : 1.0) * double(l0) : 0.0;
             const double a1 = v1 ? (n0 + q1 ? 2.0 : 1.0) * double(l1) : 0.0;
 #pragma unroll
-            for (int u = 0; u < kSdBlocks; ++u) {
+            for (int u = 0; u < kSdTiles; ++u) {
                 dmma_884(acc[u], a0, v0 ? double(t0[u]) : 0.0);
                 dmma_884(acc[u], a1, v1 ? double(t1[u]) : 0.0);
             }
@@ -179,12 +184,13 @@ __global__ void __launch_bounds__(128) sddmm_dmma_kernel(int n_block_rows, int n
         }
         if (fr < b) {
 #pragma unroll
-            for (int u = 0; u < kSdBlocks; ++u)
-                if (kb + u < ke) {
-                    double* g = grad + (int64_t(kb + u) * b + fr) * b;
+            for (int u = 0; u < kSdTiles; ++u)
 #pragma unroll
-                    for (int v = 0; v < 2; ++v)
-                        if (2 * fc + v < b) g[2 * fc + v] += scale * acc[u][v];
+                for (int v = 0; v < 2; ++v) {
+                    const int n = col0 + 8 * u + 2 * fc + v, blk = n / b;
+                    if (n < cols)
+                        grad[(int64_t(kb + blk) * b + fr) * b + (n - blk * b)] +=
+                            scale * acc[u][v];
                 }
         }
     }
@@ -199,7 +205,8 @@ int launch_sddmm(rsatb_context* ctx, const rsatb_bsr_matrix* H, int R, int n0, i
     const int used = std::min(len, n_last - n0 + 1);
     if (H->block_size >= 4 && H->block_size <= 8) {
         if (used <= 0 || H->nnz_blocks == 0) return RSATB_SUCCESS;
-        const int chunks = (std::max(1, H->max_row_blocks) + kSdBlocks - 1) / kSdBlocks;
+        const int chunks = (std::max(1, H->max_row_blocks) * H->block_size + 8 * kSdTiles - 1) /
+                           (8 * kSdTiles);
         int64_t g = (int64_t(H->n_block_rows) * chunks + 3) / 4;
         if (g > int64_t(ctx->sm_count) * 32) g = int64_t(ctx->sm_count) * 32;
         const bool pair = R % 2 == 0 && panel % 2 == 0 &&
