@@ -23,8 +23,8 @@
 //   sequences, built and read back with coalesced accesses;
 // * the contraction gives each energy k to one CTA per chunk: no atomics,
 //   the same summation order on every run;
-// * at M = 2048 (Greenwood) the row stage is one hand-written kernel after a
-//   coalesced gather: extension, 4096-point transform and contraction
+// * at M = 256, 512, 1024 and 2048 (Greenwood) the row stage is one
+//   hand-written kernel after a coalesced gather: transform and contraction
 //   without the FP64 extension buffer's round trips (greenwood_fused_kernel).
 #include "cheb_kernels.cuh"
 
@@ -515,40 +515,52 @@ __global__ void __launch_bounds__(256) greenwood_contract_kernel(int M, int64_t 
 }
 
 // ---------------------------------------------------------------------------
-// Fused Greenwood row stage for M = 2048 (a 4096-point transform): the even
-// extension, the DCT-III (the inverse 2M-point DFT of extend_kernel's
-// sequence, outputs k < M) and the contraction in one kernel, so no
-// extended sequence or transform output goes through HBM.  The transform
-// runs in FP64 for FP64 vectors and in FP32 for FP32 vectors; the products
+// Fused Greenwood row stage for M = 256, 512, 1024 and 2048: the DCT-III as the
+// M-point transform of dct3_input_kernel's sequence and the contraction in one
+// kernel, so no transform input or output goes through HBM.  The transform
+// runs in FP64, but for FP32 vectors at M = 2048 in FP32; the products
 // conj(L3) R3 and their sums are FP64 in both.
 //
-// One CTA of 256 threads transforms one sequence at a time as 16 x 16 x 16
-// (n = n0 + 16 n1 + 256 n2, k = k0 + 16 k1 + 256 k2, w = e^{2 pi i / 4096}):
-//   pass A  thread (n0, n1): 16-point DFT over n2 -> k0, times w^{(n0 + 16 n1) k0}
+// M = 16 x 16 x r (n = n0 + r n1 + 16 r n2, k = k0 + 16 k1 + 256 k2, n0, k2 < r,
+// w = e^{2 pi i / M}); 16 r threads hold a sequence, 16 values each:
+//   pass A  thread n' = n0 + r n1: 16-point DFT over n2 -> k0, times w^{n' k0}
 //   pass B  thread (n0, k0): 16-point DFT over n1 -> k1, times w^{16 n0 k1}
-//   pass C  thread (k0, k1): 16-point DFT over n0 -> k2; k < 2048 is k2 < 8
-// with the values between passes exchanged through shared memory (planes of
-// 257 entries, so the 16-byte accesses of a quarter warp fall on distinct
-// banks).  Pass A builds the extension as it loads: E_n = ph_n x_n (n < M),
-// 0 (n = M), conj(ph_{2M-n}) x_{2M-n} (n > M), ph_m = w_m e^{i pi m / 2M}.
-// Each thread keeps the left sequence's 8 outputs, transforms the right
-// sequence and accumulates conj(L3_k) R3_k for its 8 energies in FP64 over
-// the CTA's sequences (a fixed grid-stride order); fused_reduce_kernel sums
-// the CTAs in a fixed order, so results do not depend on timing.
+//   pass C  thread's 16 / r pairs (k1, k0): r-point DFT over n0 -> k2
+// exchanged through shared memory.  Strides between A and B: 17 r entries per
+// k0 (16 r written by consecutive lanes, read r at a time at a step of r);
+// between B and C: 16 r + 1 per k1 (written by consecutive lanes, read at a
+// stride of 1 modulo the banks).  Pass A forms
+//   F_n = ph_n x_n + conj(ph_{M-n}) x_{M-n},  F_0 = ph_0 x_0,
+//   ph_m = w_m e^{i pi m / 2M},
+// as it loads.  A CTA of 256 threads holds 8 / r pairs of a left and a right
+// sequence side by side; after pass C the two swap halves of their outputs, so
+// each thread accumulates conj(L3_k) R3_k for 8 energies in FP64 over the CTA's
+// pairs (a fixed grid-stride order); fused_reduce_kernel sums the partials in a
+// fixed order, so results do not depend on timing.
+//
+// Half the points of the even extension's 2M: half the work, in registers for
+// two CTAs per SM.  8,192 pairs of 2048 moments: FP32 119 us against 176 with the
+// extended transform.  At 512 and 1024 moments it replaces cuFFT's two passes
+// over HBM per side.  Bound by shared memory and issue.
 //
 // The store is moment-major (each moment's rows written coalesced by the
-// recurrence), so one sequence is 2048 values 8 or 16 bytes apiece at a
-// stride of the slot size; gather_sequences_kernel first turns a chunk of
-// consecutive sequences into sequence-major rows with a tiled transpose
-// (both sides coalesced), from which pass A reads 256 contiguous values per
-// warp instruction.
-constexpr int kFusedM = 2048;
+// recurrence), so one sequence is M values 8 or 16 bytes apiece at a stride
+// of the slot size; gather_sequences_kernel first turns a chunk of consecutive
+// sequences into sequence-major rows with a tiled transpose (both sides
+// coalesced), from which pass A reads contiguous values.
 constexpr int kFusedThreads = 256;
-constexpr int kXchPlane = 257;
-// Shared memory of the fused kernel: exchange planes, w^j (j < 1024), ph.
+
+// r for a moment count the fused stage serves, else 0.
+inline int fused_radix(int M) {
+    return M == 256 || M == 512 || M == 1024 || M == 2048 ? M / 256 : 0;
+}
+// Exchange entries of one sequence; pairs of sequences per CTA; partial sums.
+__host__ __device__ constexpr int fused_xch(int r) { return 16 * (16 * r + r); }
+__host__ __device__ constexpr int fused_pairs(int r) { return 8 / r; }
+// Shared memory: exchange, w^j (j < M / 4), ph.
 template <typename C>
-constexpr size_t fused_smem() {
-    return size_t(16 * kXchPlane + 1024 + kFusedM) * sizeof(C);
+size_t fused_smem(int r) {
+    return size_t(2 * fused_pairs(r) * fused_xch(r) + 64 * r + 256 * r) * sizeof(C);
 }
 
 // Complex arithmetic on float2 (FP32 transform) and double2 (FP64 transform).
@@ -614,11 +626,37 @@ __device__ __forceinline__ void dft16_inv(C (&v)[16]) {
 }
 __device__ __forceinline__ int dft16_at(int k) { return 4 * (k & 3) + (k >> 2); }
 
-// w^n = e^{2 pi i n / 4096} from the quarter table q[j] = w^j, j < 1024.
-template <typename C>
-__device__ __forceinline__ C twiddle4096(const C* q, int n) {
-    const C b = q[n & 1023];
-    switch ((n >> 10) & 3) {
+// r-point DFT with the + sign, r <= 16, natural order out.
+template <typename C, int r>
+__device__ __forceinline__ void dft_r_inv(C (&v)[r]) {
+    if constexpr (r == 2) {
+        const C t = c_sub(v[0], v[1]);
+        v[0] = c_add(v[0], v[1]);
+        v[1] = t;
+    } else if constexpr (r == 4) {
+        dft4_inv(v[0], v[1], v[2], v[3]);
+    } else if constexpr (r == 8) {
+        using S = typename Cx<C>::S;
+        constexpr S r2 = S(0.70710678118654752);  // cos(pi / 4)
+        C e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
+        dft4_inv(e[0], e[1], e[2], e[3]);
+        dft4_inv(o[0], o[1], o[2], o[3]);
+        o[1] = c_mul(o[1], Cx<C>::make(r2, r2));
+        o[2] = c_mul_i(o[2]);
+        o[3] = c_mul(o[3], Cx<C>::make(-r2, r2));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            v[k] = c_add(e[k], o[k]);
+            v[k + 4] = c_sub(e[k], o[k]);
+        }
+    }
+}
+
+// w^n = e^{2 pi i n / M} from the quarter table q[j] = w^j, j < M / 4.
+template <typename C, int M>
+__device__ __forceinline__ C twiddle(const C* q, int n) {
+    const C b = q[n & (M / 4 - 1)];
+    switch ((n / (M / 4)) & 3) {
         case 0: return b;
         case 1: return Cx<C>::make(-b.y, b.x);
         case 2: return Cx<C>::make(-b.x, -b.y);
@@ -661,85 +699,84 @@ __device__ __forceinline__ C load_c(const double* S, int64_t e) {
     return Cx<C>::make(typename Cx<C>::S(f.x), typename Cx<C>::S(f.y));
 }
 
-// The 8 outputs k0 + 16 k1 + 256 k2 (k2 < 8) of thread (k0, k1) for the
-// sequence whose element m is S[m + base] (complex index; sequence-major).
-template <typename C, typename T>
-__device__ __forceinline__ void fused_transform(const T* S, int64_t base, const C* qtw,
-                                                const C* ph, C* xch, C (&out)[8]) {
-    const int t = threadIdx.x;
+// The 16 outputs of thread t of a sequence whose element m is S[m]: out[j r +
+// k2] is p = k0 + 16 k1 + 256 k2 for the pair 16 k0 + k1 = t + 16 r j.  All the
+// CTA's threads run it together (xch: this sequence's exchange buffer).
+template <typename C, int r, typename T>
+__device__ __forceinline__ void fused_transform(const T* S, int t, const C* qtw, const C* ph,
+                                                C* xch, C (&out)[16]) {
+    constexpr int M = 256 * r, TPS = 16 * r;
     C v[16];
-    // pass A: thread (n0, n1) = (t % 16, t / 16) holds E_{t + 256 n2}
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
-        const int n = t + 256 * j;
-        if (j < 8) {
-            v[j] = c_mul(ph[n], load_c<C>(S, base + n));
-        } else if (n == kFusedM) {
-            v[j] = Cx<C>::make(0, 0);
-        } else {
-            const int m = 2 * kFusedM - n;
-            const C p = ph[m];
-            v[j] = c_mul(Cx<C>::make(p.x, -p.y), load_c<C>(S, base + m));
+        const int n = t + TPS * j;
+        C f = c_mul(ph[n], load_c<C>(S, n));
+        if (n != 0) {
+            const C p = ph[M - n];
+            f = c_add(f, c_mul(Cx<C>::make(p.x, -p.y), load_c<C>(S, M - n)));
         }
+        v[j] = f;
     }
     dft16_inv(v);
     {
-        const int n0 = t & 15, n1 = t >> 4;
-        const Pow16<C> tw(twiddle4096(qtw, t), twiddle4096(qtw, 4 * t));  // w^{t k0}
+        const Pow16<C> tw(twiddle<C, M>(qtw, t), twiddle<C, M>(qtw, 4 * t));  // w^{n' k0}
 #pragma unroll
-        for (int k0 = 0; k0 < 16; ++k0)
-            xch[n0 * kXchPlane + k0 * 16 + n1] = c_mul(v[dft16_at(k0)], tw(k0));
+        for (int k0 = 0; k0 < 16; ++k0) xch[k0 * 17 * r + t] = c_mul(v[dft16_at(k0)], tw(k0));
     }
     __syncthreads();
-    // pass B: thread (n0, k0) = (t % 16, t / 16)
-    {
-        const int n0 = t & 15, k0 = t >> 4;
+    const int n0 = t % r, kb0 = t / r;
 #pragma unroll
-        for (int n1 = 0; n1 < 16; ++n1) v[n1] = xch[n0 * kXchPlane + k0 * 16 + n1];
-        dft16_inv(v);
-        const Pow16<C> tw(twiddle4096(qtw, 16 * n0), twiddle4096(qtw, 64 * n0));  // w^{16 n0 k1}
-        __syncthreads();
+    for (int n1 = 0; n1 < 16; ++n1) v[n1] = xch[kb0 * 17 * r + n0 + r * n1];
+    dft16_inv(v);
+    __syncthreads();
+    if constexpr (r > 1) {
+        const Pow16<C> tw(twiddle<C, M>(qtw, 16 * n0), twiddle<C, M>(qtw, 64 * n0));
 #pragma unroll
         for (int k1 = 0; k1 < 16; ++k1)
-            xch[k0 * kXchPlane + k1 * 16 + n0] = c_mul(v[dft16_at(k1)], tw(k1));
+            xch[k1 * (16 * r + 1) + t] = c_mul(v[dft16_at(k1)], tw(k1));
+    } else {
+#pragma unroll
+        for (int k1 = 0; k1 < 16; ++k1) xch[k1 * (16 * r + 1) + t] = v[dft16_at(k1)];
     }
     __syncthreads();
-    // pass C: thread (k0, k1) = (t % 16, t / 16)
-    {
-        const int k0 = t & 15, k1 = t >> 4;
 #pragma unroll
-        for (int n0 = 0; n0 < 16; ++n0) v[n0] = xch[k0 * kXchPlane + k1 * 16 + n0];
-        dft16_inv(v);
+    for (int j = 0; j < 16 / r; ++j) {
+        const int pi = t + TPS * j, k1 = pi & 15, k0 = pi >> 4;
+        C u[r];
 #pragma unroll
-        for (int k2 = 0; k2 < 8; ++k2) out[k2] = v[dft16_at(k2)];
+        for (int q = 0; q < r; ++q) u[q] = xch[k1 * (16 * r + 1) + k0 * r + q];
+        dft_r_inv<C, r>(u);
+#pragma unroll
+        for (int q = 0; q < r; ++q) out[j * r + q] = u[q];
     }
-    __syncthreads();  // xch is rewritten by the next transform
+    __syncthreads();  // xch is rewritten
 }
 
-// The tables of the transform: tab[j] = w^j (j < 1024), tab[1024 + m] = ph_m.
-__global__ void fused_tables_kernel(const double* w, double2* tab) {
+// The tables of the transform: tab[j] = w^j (j < M / 4), tab[M / 4 + m] = ph_m.
+__global__ void fused_tables_kernel(int M, const double* w, double2* tab) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     double s, c;
-    if (i < 1024) {
-        sincospi(double(i) / 2048.0, &s, &c);  // w^j = e^{2 pi i j / 4096}
+    if (i < M / 4) {
+        sincospi(2.0 * double(i) / double(M), &s, &c);
         tab[i] = make_double2(c, s);
-    } else if (i < 1024 + kFusedM) {
-        const int m = i - 1024;
-        sincospi(double(m) / (2.0 * kFusedM), &s, &c);  // e^{i pi m / 2M}
+    } else if (i < M / 4 + M) {
+        const int m = i - M / 4;
+        sincospi(double(m) / (2.0 * double(M)), &s, &c);  // e^{i pi m / 2M}
         tab[i] = make_double2(w[m] * c, w[m] * s);
     }
 }
 
-// Tq[side][i][m] = S_side[m * slot + q0 + i] for i < nqc (complex entries):
-// 32 x 32 tiles through shared memory, blockIdx.z the side (left, right).
+// Tq[side][i][m] = S_side[m * slot + q0 + i] for i < nqc (complex entries, M a
+// multiple of 32): 32 x 32 tiles through shared memory, blockIdx.z the side
+// (left, right).
 template <typename T>
-__global__ void __launch_bounds__(256) gather_sequences_kernel(int64_t q0, int64_t nqc,
+__global__ void __launch_bounds__(256) gather_sequences_kernel(int M, int64_t q0, int64_t nqc,
                                                                int64_t slot, const T* SL,
                                                                const T* SR, T* Tq) {
     using C = typename std::conditional<std::is_same<T, float>::value, float2, double2>::type;
     __shared__ C tile[32][33];
     const C* S = reinterpret_cast<const C*>(blockIdx.z ? SR : SL);
-    C* out = reinterpret_cast<C*>(Tq) + int64_t(blockIdx.z) * nqc * kFusedM;
+    C* out = reinterpret_cast<C*>(Tq) + int64_t(blockIdx.z) * nqc * M;
     const int64_t i0 = int64_t(blockIdx.x) * 32;
     const int m0 = blockIdx.y * 32;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -752,63 +789,124 @@ __global__ void __launch_bounds__(256) gather_sequences_kernel(int64_t q0, int64
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         const int64_t i = i0 + ty + 8 * r;
-        if (i < nqc) out[i * kFusedM + m0 + tx] = tile[tx][ty + 8 * r];
+        if (i < nqc) out[i * M + m0 + tx] = tile[tx][ty + 8 * r];
     }
 }
 
-// Gathered sequences i < nqc of one chunk (Tq, left then right), transform
-// in the precision of C; partial[cta][k] += sum over the CTA's sequences of
-// conj(L3_k) R3_k, the products and the sums in FP64.  Two CTAs per SM for
-// the FP32 transform (half the registers and shared memory), one for FP64.
-template <typename T, typename C>
-__global__ void __launch_bounds__(kFusedThreads, sizeof(C) == 8 ? 2 : 1)
+// Gathered sequences i < nqc of one chunk (Tq, left then right), transform in
+// the precision of C; partial[cta][pair][p] += sum over the pair's sequences of
+// conj(L3) R3, the products and the sums in FP64.
+template <typename T, typename C, int r>
+__global__ void __launch_bounds__(kFusedThreads, 2)
     greenwood_fused_kernel(int64_t nqc, const T* Tq, const double2* tab, double2* partial) {
+    constexpr int M = 256 * r, TPS = 16 * r, P = fused_pairs(r);
     extern __shared__ __align__(16) unsigned char fsm_raw[];
-    C* xch = reinterpret_cast<C*>(fsm_raw);
-    C* qtw = xch + 16 * kXchPlane;
-    C* ph = qtw + 1024;
-    for (int j = threadIdx.x; j < 1024 + kFusedM; j += blockDim.x)
+    C* xch0 = reinterpret_cast<C*>(fsm_raw);
+    C* qtw = xch0 + 2 * P * fused_xch(r);
+    C* ph = qtw + M / 4;
+    for (int j = threadIdx.x; j < M / 4 + M; j += blockDim.x)
         qtw[j] = Cx<C>::make(typename Cx<C>::S(tab[j].x), typename Cx<C>::S(tab[j].y));
     __syncthreads();
+    const int seq = threadIdx.x / TPS, t = threadIdx.x - seq * TPS;
+    const int side = seq & 1, pair = seq >> 1;  // left and right side by side
+    C* mine = xch0 + seq * fused_xch(r);
+    C* other = xch0 + (seq ^ 1) * fused_xch(r);
     double2 acc[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[i] = make_double2(0.0, 0.0);
-    const int64_t right = nqc * kFusedM;
-    for (int64_t i = blockIdx.x; i < nqc; i += gridDim.x) {
-        C l3[8], r3[8];
-        fused_transform(Tq, i * kFusedM, qtw, ph, xch, l3);
-        fused_transform(Tq, right + i * kFusedM, qtw, ph, xch, r3);
+    const int64_t step = int64_t(gridDim.x) * P;
+    // The same number of rounds for every pair of a CTA (barriers inside);
+    // pairs past the end transform the last sequence and add nothing.
+    for (int64_t i0 = int64_t(blockIdx.x) * P; i0 < nqc; i0 += step) {
+        const int64_t i = i0 + pair;
+        const bool live = i < nqc;
+        C out[16];
+        fused_transform<C, r>(Tq + 2 * (side * nqc + (live ? i : nqc - 1)) * M, t, qtw, ph, mine,
+                              out);
+        // The left thread gives its outputs 8.. and takes the right's 0..7.
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const double lx = l3[j].x, ly = l3[j].y, rx = r3[j].x, ry = r3[j].y;
-            acc[j].x += lx * rx + ly * ry;  // conj(L3) R3
-            acc[j].y += lx * ry - ly * rx;
+        for (int j = 0; j < 8; ++j)
+            mine[j * TPS + t] = Cx<C>::make(side ? out[j].x : out[j + 8].x,
+                                            side ? out[j].y : out[j + 8].y);
+        __syncthreads();
+        if (live) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const C o = other[j * TPS + t];
+                const double lx = side ? o.x : out[j].x, ly = side ? o.y : out[j].y;
+                const double rx = side ? out[j + 8].x : o.x, ry = side ? out[j + 8].y : o.y;
+                acc[j].x += lx * rx + ly * ry;  // conj(L3) R3
+                acc[j].y += lx * ry - ly * rx;
+            }
         }
+        __syncthreads();
     }
-    double2* p = partial + int64_t(blockIdx.x) * kFusedM + threadIdx.x;
+    double2* p = partial + (int64_t(blockIdx.x) * P + pair) * M;
 #pragma unroll
-    for (int k2 = 0; k2 < 8; ++k2) p[256 * k2] = make_double2(p[256 * k2].x + acc[k2].x,
-                                                              p[256 * k2].y + acc[k2].y);
+    for (int j = 0; j < 8; ++j) {
+        const int o = side ? j + 8 : j;
+        const int pi = t + TPS * (o / r), e = (pi >> 4) + 16 * (pi & 15) + 256 * (o % r);
+        p[e] = make_double2(p[e].x + acc[j].x, p[e].y + acc[j].y);
+    }
 }
 
-// K[k][comp] += sum over the n_cta partials (in CTA order) / max(1e-14, 1 - eps_k^2).
-__global__ void fused_reduce_kernel(int n_cta, const double2* partial, int comp, double* K) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= kFusedM) return;
+// K[k][comp] += sum over the n_part partials / max(1e-14, 1 - eps_k^2), one CTA
+// per transform output, a fixed order.
+__global__ void __launch_bounds__(128) fused_reduce_kernel(int M, int n_part,
+                                                           const double2* partial, int comp,
+                                                           double* K) {
+    __shared__ double2 red[128];
     double re = 0.0, im = 0.0;
-    for (int c = 0; c < n_cta; ++c) {
-        const double2 p = partial[int64_t(c) * kFusedM + k];
+    for (int c = threadIdx.x; c < n_part; c += blockDim.x) {
+        const double2 p = partial[int64_t(c) * M + blockIdx.x];
         re += p.x;
         im += p.y;
     }
-    const double eps = cos(M_PI * (double(k) + 0.5) / double(kFusedM));
+    red[threadIdx.x] = make_double2(re, im);
+    __syncthreads();
+    for (int w = 64; w > 0; w >>= 1) {
+        if (threadIdx.x < w) {
+            red[threadIdx.x].x += red[threadIdx.x + w].x;
+            red[threadIdx.x].y += red[threadIdx.x + w].y;
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x) return;
+    const int k = dct3_energy(M, blockIdx.x);
+    const double eps = cos(M_PI * (double(k) + 0.5) / double(M));
     const double wden = 1.0 - eps * eps;
     const double inv = 1.0 / (wden > 1e-14 ? wden : 1e-14);
-    K[2 * (int64_t(k) * 6 + comp)] += re * inv;
-    K[2 * (int64_t(k) * 6 + comp) + 1] += im * inv;
+    K[2 * (int64_t(k) * 6 + comp)] += red[0].x * inv;
+    K[2 * (int64_t(k) * 6 + comp) + 1] += red[0].y * inv;
 }
 
-// The fused row stage serves Greenwood at M = 2048 unless RSATB_FFTCHEB_FUSED=0.
+// One chunk of the fused stage: grid CTAs (returned to the caller for sizing
+// through fused_grid) of the transform's type and radix.
+template <typename T, typename C, int r>
+int fused_launch(rsatb_context* ctx, int grid, int64_t n, const T* Tq, const double2* tab,
+                 double2* partial) {
+    RSATB_CUDA_TRY(cudaFuncSetAttribute(greenwood_fused_kernel<T, C, r>,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        int(fused_smem<C>(r))));
+    greenwood_fused_kernel<T, C, r>
+        <<<grid, kFusedThreads, fused_smem<C>(r), ctx->stream>>>(n, Tq, tab, partial);
+    RSATB_LAUNCH_CHECK(ctx);
+    return RSATB_SUCCESS;
+}
+
+template <typename T, typename C>
+int fused_launch_r(rsatb_context* ctx, int r, int grid, int64_t n, const T* Tq,
+                   const double2* tab, double2* partial) {
+    switch (r) {
+        case 1: return fused_launch<T, C, 1>(ctx, grid, n, Tq, tab, partial);
+        case 2: return fused_launch<T, C, 2>(ctx, grid, n, Tq, tab, partial);
+        case 4: return fused_launch<T, C, 4>(ctx, grid, n, Tq, tab, partial);
+        default: return fused_launch<T, C, 8>(ctx, grid, n, Tq, tab, partial);
+    }
+}
+
+// The fused row stage serves Greenwood at fused_radix's moment counts unless
+// RSATB_FFTCHEB_FUSED=0.
 bool fused_enabled() {
     const char* s = std::getenv("RSATB_FFTCHEB_FUSED");
     return !(s && s[0] == '0');
@@ -1030,11 +1128,12 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
                          workspace, fixed, store_per_brow);
     // FFT chunk: rows whose 2 x (2M x 3 rows R) double2 extensions fit a
     // quarter of what remains after the fixed buffers.  The fused row stage
-    // (Greenwood, M = 2048) needs only its gathered chunk of up to 8,192
+    // (Greenwood, fused_radix) needs only its gathered chunk of up to 8,192
     // sequence pairs, and the store takes the rest (larger sections: fewer
     // passes of the recurrence).
     const size_t avail = workspace - fixed;
-    const bool fused = !bastin && M == kFusedM && fused_enabled();
+    const int radix = bastin ? 0 : fused_radix(M);
+    const bool fused = radix && fused_enabled();
     const size_t fused_chunk_bytes = 2 * size_t(8192) * size_t(M) * cplx;
     const size_t fft_budget =
         fused ? std::max(2 * size_t(M) * cplx, std::min(avail / 4, fused_chunk_bytes))
@@ -1123,13 +1222,15 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
     }
     RSATB_CUDA_TRY(cudaMemsetAsync(K, 0, size_t(M) * 12 * sizeof(double), st));
 
-    // Fused row stage (Greenwood, M = 2048): one CTA per SM, partial sums
-    // per CTA and energy; chunks of fused_qc sequences gathered into the
-    // extension buffer (sequence-major, both sides).
-    // FP32 vectors take the FP32 transform (FP64 products and sums) unless
-    // RSATB_FFTCHEB_FP64=1; FP64 vectors the FP64 one.
-    const bool fused32 = fused && std::is_same<T, float>::value && !fused_fp64_forced();
-    const int fused_grid = ctx->sm_count * (fused32 ? 2 : 1);
+    // Fused row stage: two CTAs per SM, partial sums per CTA, pair of sequences
+    // and energy; chunks of fused_qc sequences gathered into the extension
+    // buffer (sequence-major, both sides).  FP32 vectors take the FP32
+    // transform at M = 2048 (FP64 products and sums) unless
+    // RSATB_FFTCHEB_FP64=1; every other case the FP64 one.
+    const bool fused32 = fused && M == 2048 && std::is_same<T, float>::value &&
+                         !fused_fp64_forced();
+    const int fused_grid = ctx->sm_count * 2;
+    const int n_part = fused ? fused_grid * fused_pairs(radix) : 0;
     int64_t fused_qc = std::max<int64_t>(
         1, std::min<int64_t>(8192, int64_t(e_bytes / (2 * size_t(M) * cplx))));
     if (const char* cap = std::getenv("RSATB_FFTCHEB_CHUNK")) {  // smaller chunks (tests)
@@ -1138,18 +1239,11 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
     }
     DevBuf bPart, bTab;
     if (fused) {
-        RSATB_TRY(bPart.alloc(size_t(fused_grid) * kFusedM * sizeof(double2)));
-        RSATB_TRY(bTab.alloc(size_t(1024 + kFusedM) * sizeof(double2)));
-        fused_tables_kernel<<<(1024 + kFusedM) / 256, 256, 0, st>>>(bWts.as<double>(),
-                                                                    bTab.as<double2>());
+        RSATB_TRY(bPart.alloc(size_t(n_part) * M * sizeof(double2)));
+        RSATB_TRY(bTab.alloc(size_t(M / 4 + M) * sizeof(double2)));
+        fused_tables_kernel<<<(M / 4 + M + 255) / 256, 256, 0, st>>>(M, bWts.as<double>(),
+                                                                     bTab.as<double2>());
         RSATB_LAUNCH_CHECK(ctx);
-        RSATB_CUDA_TRY(cudaFuncSetAttribute(greenwood_fused_kernel<T, double2>,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            int(fused_smem<double2>())));
-        if constexpr (std::is_same<T, float>::value)
-            RSATB_CUDA_TRY(cudaFuncSetAttribute(greenwood_fused_kernel<T, float2>,
-                                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                int(fused_smem<float2>())));
     }
 
     // cuFFT plans: full chunks and the last, shorter chunk of a section.
@@ -1318,39 +1412,38 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
         cudaEventElapsedTime(&t, ev0, ev1);
         rec_ms += t;
 
-        // Row stage: fused at M = 2048 (Greenwood), else in chunks of rows
-        // through the extension, cuFFT and the contraction.
+        // Row stage: fused (Greenwood, fused_radix), else in chunks of rows
+        // through the transform input, cuFFT and the contraction.
         RSATB_CUDA_TRY(cudaEventRecord(ev0, st));
         if (fused) {
             const int64_t per_axis = rows * R;
             T* Tq = reinterpret_cast<T*>(EL);
             for (int a = 0; a < 3; ++a) {
-                RSATB_CUDA_TRY(cudaMemsetAsync(
-                    bPart.p, 0, size_t(fused_grid) * kFusedM * sizeof(double2), st));
+                RSATB_CUDA_TRY(
+                    cudaMemsetAsync(bPart.p, 0, size_t(n_part) * M * sizeof(double2), st));
                 for (int64_t i0 = 0; i0 < per_axis; i0 += fused_qc) {
                     const int64_t n = std::min<int64_t>(fused_qc, per_axis - i0);
-                    const dim3 gg(unsigned((n + 31) / 32), kFusedM / 32, 2);
-                    gather_sequences_kernel<T><<<gg, 256, 0, st>>>(int64_t(a) * per_axis + i0, n,
-                                                                   sslot, SL, SR, Tq);
+                    const dim3 gg(unsigned((n + 31) / 32), M / 32, 2);
+                    gather_sequences_kernel<T><<<gg, 256, 0, st>>>(
+                        M, int64_t(a) * per_axis + i0, n, sslot, SL, SR, Tq);
                     RSATB_LAUNCH_CHECK(ctx);
                     bool done = false;
                     if constexpr (std::is_same<T, float>::value) {
                         if (fused32) {
-                            greenwood_fused_kernel<T, float2>
-                                <<<fused_grid, kFusedThreads, fused_smem<float2>(), st>>>(
-                                    n, Tq, bTab.as<double2>(), bPart.as<double2>());
+                            RSATB_TRY((fused_launch<T, float2, 8>(ctx, fused_grid, n, Tq,
+                                                                  bTab.as<double2>(),
+                                                                  bPart.as<double2>())));
                             done = true;
                         }
                     }
                     if (!done)
-                        greenwood_fused_kernel<T, double2>
-                            <<<fused_grid, kFusedThreads, fused_smem<double2>(), st>>>(
-                                n, Tq, bTab.as<double2>(), bPart.as<double2>());
-                    RSATB_LAUNCH_CHECK(ctx);
+                        RSATB_TRY((fused_launch_r<T, double2>(ctx, radix, fused_grid, n, Tq,
+                                                              bTab.as<double2>(),
+                                                              bPart.as<double2>())));
                     ++chunks;
                 }
-                fused_reduce_kernel<<<kFusedM / 256, 256, 0, st>>>(
-                    fused_grid, bPart.as<double2>(), a == 0 ? 0 : (a == 1 ? 3 : 5), K);
+                fused_reduce_kernel<<<M, 128, 0, st>>>(
+                    M, n_part, bPart.as<double2>(), a == 0 ? 0 : (a == 1 ? 3 : 5), K);
                 RSATB_LAUNCH_CHECK(ctx);
             }
         }
