@@ -72,6 +72,18 @@ struct rsatb_context {
     std::string kpm_graph_key;
     std::string kpm_seen_key;
     int64_t kpm_graph_launches = 0;
+    // The transport's workspace, kept between calls up to kKeepWorkShare of the
+    // device's memory (larger ones are the call's own), and the last two cuFFT
+    // plans it made (their work areas lie in the workspace).
+    void* work = nullptr;
+    size_t work_bytes = 0;
+    struct FftPlan {
+        int handle = 0;
+        int n = 0;
+        int64_t batch = 0;  // 0: empty
+        size_t work = 0;
+    } fft[2];
+    int fft_next = 0;
     // Pinned host staging (grow-only) for small asynchronous read-backs.
     void* pinned = nullptr;
     size_t pinned_bytes = 0;

@@ -1,6 +1,8 @@
 // Context, memory and error entry points of the C ABI.
 #include "common.cuh"
 
+#include <cufft.h>
+
 #include <mutex>
 #include <vector>
 
@@ -154,6 +156,9 @@ int rsatb_ctx_destroy(rsatb_ctx_t ctx) {
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     if (ctx->scratch) cudaFree(ctx->scratch);
+    if (ctx->work) cudaFree(ctx->work);
+    for (auto& f : ctx->fft)
+        if (f.batch) cufftDestroy(f.handle);
     if (ctx->counters) cudaFree(ctx->counters);
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
     if (ctx->kpm_graph) cudaGraphExecDestroy(ctx->kpm_graph);

@@ -939,13 +939,97 @@ struct DevBuf {
     }
 };
 
-struct Plan {
-    cufftHandle h = 0;
-    bool made = false;
-    ~Plan() {
-        if (made) cufftDestroy(h);
+// Device memory of one call: every buffer is a piece of one block, the
+// context's kept one when the call needs at most 1/16 of the device's memory,
+// else one allocation released at the end.  (Ten cudaMalloc / cudaFree pairs
+// per call cost 20 ms at 11 GB, 4 ms at 0.5 GB.)
+constexpr size_t kKeepWorkShare = 16;
+
+class Arena {
+  public:
+    size_t reserve(size_t bytes) {
+        const size_t at = total_;
+        total_ += (std::max<size_t>(bytes, 16) + 255) & ~size_t(255);
+        return at;
     }
+    int commit(rsatb_context* ctx) {
+        size_t free_b = 0, total_b = 0;
+        if (ctx->work_bytes < total_) {
+            RSATB_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
+            if (total_ > total_b / kKeepWorkShare) {
+                // The kept block may be what is missing.
+                cudaError_t e = cudaMalloc(&own_.p, total_);
+                if (e == cudaErrorMemoryAllocation && ctx->work) {
+                    cudaGetLastError();
+                    RSATB_TRY(drop(ctx));
+                    e = cudaMalloc(&own_.p, total_);
+                }
+                RSATB_CUDA_TRY(e);
+                base_ = own_.as<char>();
+                return RSATB_SUCCESS;
+            }
+            RSATB_TRY(drop(ctx));
+            RSATB_CUDA_TRY(cudaMalloc(&ctx->work, total_));
+            ctx->work_bytes = total_;
+        }
+        base_ = static_cast<char*>(ctx->work);
+        return RSATB_SUCCESS;
+    }
+    template <typename T>
+    T* at(size_t offset) const {
+        return reinterpret_cast<T*>(base_ + offset);
+    }
+
+  private:
+    static int drop(rsatb_context* ctx) {
+        if (!ctx->work) return RSATB_SUCCESS;
+        RSATB_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+        void* p = ctx->work;
+        ctx->work = nullptr;
+        ctx->work_bytes = 0;
+        RSATB_CUDA_TRY(cudaFree(p));
+        return RSATB_SUCCESS;
+    }
+    size_t total_ = 0;
+    char* base_ = nullptr;
+    DevBuf own_;
 };
+
+// The context's inverse Z2Z plan of `batch` interleaved sequences of n points
+// (stride batch), made at its first use; *work is its work area's size.
+int fft_plan(rsatb_context* ctx, int n, int64_t batch, cufftHandle* out, size_t* work) {
+    for (auto& f : ctx->fft)
+        if (f.batch == batch && f.n == n) {
+            *out = f.handle;
+            *work = f.work;
+            return RSATB_SUCCESS;
+        }
+    auto& f = ctx->fft[ctx->fft_next];
+    ctx->fft_next ^= 1;
+    if (f.batch) {
+        f.batch = 0;
+        cufftDestroy(f.handle);
+    }
+    cufftHandle h = 0;
+    RSATB_CUFFT_TRY(cufftCreate(&h));
+    size_t w = 0;
+    int nn = n;
+    cufftResult r = cufftSetAutoAllocation(h, 0);
+    if (r == CUFFT_SUCCESS)
+        r = cufftMakePlanMany(h, 1, &nn, &nn, int(batch), 1, &nn, int(batch), 1, CUFFT_Z2Z,
+                              int(batch), &w);
+    if (r != CUFFT_SUCCESS) {
+        cufftDestroy(h);
+        return set_error(RSATB_CUDA_ERROR, "cufftMakePlanMany failed (cufftResult %d)", int(r));
+    }
+    f.handle = h;
+    f.n = n;
+    f.batch = batch;
+    f.work = w;
+    *out = h;
+    *work = w;
+    return RSATB_SUCCESS;
+}
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
@@ -1087,21 +1171,23 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
     if (workspace == 0) {
         size_t free_b = 0, total_b = 0;
         RSATB_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-        workspace = free_b / 10 * 8;
+        workspace = (free_b + ctx->work_bytes) / 10 * 8;  // the kept block is reused
     }
     // One launch per moment (moment_kernel) where the four matrices allow it
     // and its buffers (two panels, the start, the packed values) are no larger
     // than the separate launches' or small in the workspace; RSATB_FFTCHEB_MOMENT=0
     // keeps the separate launches.
-    DevBuf bPan, bInit, bWgt;
+    T* wgt = nullptr;  // in the context's scratch
     const int64_t nnz = c.op->H->nnz_blocks;
     const size_t fixed_m =
         size_t(N) * cplx * 3 * 4 * R + 4 * size_t(nnz) * sizeof(T) + sizeof(int) + 256;
     bool one_launch = moment_enabled() && moment_matrices_ok(c, V, R) &&
                       fixed_m <= std::max(fixed, workspace / 8);
     if (one_launch) {
-        RSATB_TRY(bWgt.alloc(4 * size_t(nnz) * sizeof(T) + 256));
-        int* d_differs = reinterpret_cast<int*>(bWgt.as<T>() + 4 * nnz);
+        void* sc = nullptr;
+        RSATB_TRY(ctx_scratch(ctx, 4 * size_t(nnz) * sizeof(T) + 256, &sc));
+        wgt = static_cast<T*>(sc);
+        int* d_differs = reinterpret_cast<int*>(wgt + 4 * nnz);
         RSATB_CUDA_TRY(cudaMemsetAsync(d_differs, 0, sizeof(int), st));
         const rsatb_bsr_matrix* H = c.op->H;
         pack_weights_kernel<T><<<grid_for(std::max<int64_t>(nnz, N + 1), ctx->sm_count), 256, 0,
@@ -1109,18 +1195,16 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
             N, nnz, H->row_ptr, H->col_ind, static_cast<const T*>(H->values), V[0]->row_ptr,
             V[0]->col_ind, static_cast<const T*>(V[0]->values), V[1]->row_ptr, V[1]->col_ind,
             static_cast<const T*>(V[1]->values), V[2]->row_ptr, V[2]->col_ind,
-            static_cast<const T*>(V[2]->values), bWgt.as<T>(), d_differs);
+            static_cast<const T*>(V[2]->values), wgt, d_differs);
         RSATB_LAUNCH_CHECK(ctx);
         int differs = 0;
         RSATB_CUDA_TRY(cudaMemcpyAsync(&differs, d_differs, sizeof(int), cudaMemcpyDeviceToHost,
                                        st));
         RSATB_CUDA_TRY(cudaStreamSynchronize(st));
-        if (differs) {
+        if (differs)
             one_launch = false;
-            bWgt.release();
-        } else {
+        else
             fixed = fixed_m;
-        }
     }
     if (workspace <= fixed + store_per_brow)
         return set_error(RSATB_OUT_OF_MEMORY,
@@ -1137,7 +1221,7 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
     const size_t fused_chunk_bytes = 2 * size_t(8192) * size_t(M) * cplx;
     const size_t fft_budget =
         fused ? std::max(2 * size_t(M) * cplx, std::min(avail / 4, fused_chunk_bytes))
-              : avail / 4;
+              : std::min(avail / 4, size_t(2) << 30);
     const size_t fft_per_row =
         2 * size_t(n_pts) * 3 * R * sizeof(double2) * 2;  // + cuFFT work
     int64_t chunk_rows = int64_t(fft_budget / fft_per_row);
@@ -1155,56 +1239,83 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
     if (chunk_rows > sec_brows * b) chunk_rows = sec_brows * b;
 
     // Buffers.
-    DevBuf bJ, bRinit, bR, bL, bU, bW, bS, bE, bK, bWts;
+    Arena mem;
     const size_t panel = size_t(N) * 8 * R;  // reals of one moment_kernel panel
-    if (one_launch) {
-        RSATB_TRY(bPan.alloc(2 * panel * sizeof(T)));
-        RSATB_TRY(bInit.alloc(panel * sizeof(T)));
-    } else {
-        RSATB_TRY(bJ.alloc(size_t(N) * 3 * R * cplx));
-        RSATB_TRY(bRinit.alloc(size_t(N) * 3 * R * cplx));
-        RSATB_TRY(bR.alloc(size_t(N) * 3 * 3 * R * cplx));
-        RSATB_TRY(bL.alloc(size_t(N) * 3 * R * cplx));
-    }
-    if (c.sandwich) {
-        RSATB_TRY(bU.alloc(size_t(N) * 3 * R * cplx));
-        RSATB_TRY(bW.alloc(size_t(N) * 3 * R * cplx));
-    }
+    const size_t v1 = size_t(N) * R * cplx;  // bytes of one N x R panel
     const int64_t sec_rows_max = sec_brows * b;
     const int64_t slot = 3 * sec_rows_max * R;  // complex entries per moment slot
-    RSATB_TRY(bS.alloc(2 * size_t(M) * slot * cplx));
     const int64_t nq_max = 3 * chunk_rows * R;
-    const size_t e_bytes =
-        fused ? fft_budget : 2 * size_t(n_pts) * nq_max * sizeof(double2);
-    RSATB_TRY(bE.alloc(e_bytes));
-    RSATB_TRY(bK.alloc(size_t(M) * 12 * sizeof(double)));
-    RSATB_TRY(bWts.alloc(size_t(M) * sizeof(double)));
-    DevBuf bPw;
-    if (bastin) RSATB_TRY(bPw.alloc(2 * size_t(M) * sizeof(double2)));
+    const size_t e_bytes = fused ? fft_budget : 2 * size_t(n_pts) * nq_max * sizeof(double2);
+    const size_t oPan = one_launch ? mem.reserve(2 * panel * sizeof(T)) : 0;
+    const size_t oInit = one_launch ? mem.reserve(panel * sizeof(T)) : 0;
+    const size_t oJ = one_launch ? 0 : mem.reserve(3 * v1);
+    const size_t oRinit = one_launch ? 0 : mem.reserve(3 * v1);
+    const size_t oR = one_launch ? 0 : mem.reserve(9 * v1);
+    const size_t oL = one_launch ? 0 : mem.reserve(3 * v1);
+    const size_t oU = c.sandwich ? mem.reserve(3 * v1) : 0;
+    const size_t oW = c.sandwich ? mem.reserve(3 * v1) : 0;
+    const size_t oS = mem.reserve(2 * size_t(M) * slot * cplx);
+    const size_t oE = mem.reserve(e_bytes);
+    const size_t oK = mem.reserve(size_t(M) * 12 * sizeof(double));
+    const size_t oWts = mem.reserve(size_t(M) * sizeof(double));
+    const size_t oPw = bastin ? mem.reserve(2 * size_t(M) * sizeof(double2)) : 0;
+    // Fused row stage: two CTAs per SM, partial sums per CTA, pair of sequences
+    // and energy; chunks of fused_qc sequences gathered into the extension
+    // buffer (sequence-major, both sides).  FP32 vectors take the FP32
+    // transform at M = 2048 (FP64 products and sums) unless
+    // RSATB_FFTCHEB_FP64=1; every other case the FP64 one.
+    const bool fused32 = fused && M == 2048 && std::is_same<T, float>::value &&
+                         !fused_fp64_forced();
+    const int fused_grid = ctx->sm_count * 2;
+    const int n_part = fused ? fused_grid * fused_pairs(radix) : 0;
+    const size_t oPart = fused ? mem.reserve(size_t(n_part) * M * sizeof(double2)) : 0;
+    const size_t oTab = fused ? mem.reserve(size_t(M / 4 + M) * sizeof(double2)) : 0;
+    // cuFFT's work area, for the chunk sizes of a full section.
+    const int fft_n = bastin ? 2 * M : M;
+    size_t fft_work = 0;
+    if (!fused) {
+        cufftHandle h = 0;
+        for (const int64_t r : {sec_rows_max % chunk_rows, chunk_rows}) {
+            size_t w = 0;
+            if (r) RSATB_TRY(fft_plan(ctx, fft_n, 3 * r * R, &h, &w));
+            fft_work = std::max(fft_work, w);
+        }
+    }
+    const size_t oFft = mem.reserve(fft_work);
+    DevBuf extra_work;  // a last, shorter section's plan may want more
+    RSATB_TRY(mem.commit(ctx));
+    void* const u_scr = c.sandwich ? mem.at<void>(oU) : nullptr;
+    void* const w_scr = c.sandwich ? mem.at<void>(oW) : nullptr;
+    T* const pan0 = mem.at<T>(oPan);
+    T* const start = mem.at<T>(oInit);
+    double* const d_wts = mem.at<double>(oWts);
+    double2* const d_pw = mem.at<double2>(oPw);
+    double2* const d_part = mem.at<double2>(oPart);
+    double2* const d_tab = mem.at<double2>(oTab);
     T* J[3];
-    for (int a = 0; a < 3; ++a) J[a] = bJ.as<T>() + size_t(a) * N * 2 * R;
-    T* rinit = bRinit.as<T>();
+    for (int a = 0; a < 3; ++a) J[a] = mem.at<T>(oJ) + size_t(a) * N * 2 * R;
+    T* rinit = mem.at<T>(oRinit);
     T* r[3];
     T* l[3];
     for (int i = 0; i < 3; ++i) {
-        r[i] = bR.as<T>() + size_t(i) * N * 6 * R;
-        l[i] = bL.as<T>() + size_t(i) * N * 2 * R;
+        r[i] = mem.at<T>(oR) + size_t(i) * N * 6 * R;
+        l[i] = mem.at<T>(oL) + size_t(i) * N * 2 * R;
     }
-    T* SL = bS.as<T>();
+    T* SL = mem.at<T>(oS);
     T* SR = SL + 2 * size_t(M) * slot;
-    double2* EL = bE.as<double2>();
+    double2* EL = mem.at<double2>(oE);
     double2* ER = EL + size_t(M) * nq_max;
     // Bastin: phi1 and phi2 of both sides.
     double2* EL1 = EL;
     double2* ER1 = EL1 + 2 * size_t(M) * nq_max;
     double2* EL2 = ER1 + 2 * size_t(M) * nq_max;
     double2* ER2 = EL2 + 2 * size_t(M) * nq_max;
-    double* K = bK.as<double>();
+    double* K = mem.at<double>(oK);
 
     std::vector<double> g(M), wts(M);
     kpm_kernel_weights(kernel, M, g.data());
     for (int m = 0; m < M; ++m) wts[m] = g[m] / M_PI;  // phi3_weight (fftcheb_transport.hpp)
-    RSATB_CUDA_TRY(cudaMemcpyAsync(bWts.p, wts.data(), M * sizeof(double),
+    RSATB_CUDA_TRY(cudaMemcpyAsync(d_wts, wts.data(), M * sizeof(double),
                                    cudaMemcpyHostToDevice, st));
     // Bastin phase weights (fftcheb_transport.hpp:302-310): phase_weight[m] =
     // 2 g_m / (pi (1 + [m == 0])) e^{i pi m / 2M}, phase_weight_m = m times it.
@@ -1217,59 +1328,21 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
             pw[m] = make_double2(coeff * std::cos(th), coeff * std::sin(th));
             pw[M + m] = make_double2(pw[m].x * double(m), pw[m].y * double(m));
         }
-        RSATB_CUDA_TRY(cudaMemcpyAsync(bPw.p, pw.data(), pw.size() * sizeof(double2),
+        RSATB_CUDA_TRY(cudaMemcpyAsync(d_pw, pw.data(), pw.size() * sizeof(double2),
                                        cudaMemcpyHostToDevice, st));
     }
     RSATB_CUDA_TRY(cudaMemsetAsync(K, 0, size_t(M) * 12 * sizeof(double), st));
 
-    // Fused row stage: two CTAs per SM, partial sums per CTA, pair of sequences
-    // and energy; chunks of fused_qc sequences gathered into the extension
-    // buffer (sequence-major, both sides).  FP32 vectors take the FP32
-    // transform at M = 2048 (FP64 products and sums) unless
-    // RSATB_FFTCHEB_FP64=1; every other case the FP64 one.
-    const bool fused32 = fused && M == 2048 && std::is_same<T, float>::value &&
-                         !fused_fp64_forced();
-    const int fused_grid = ctx->sm_count * 2;
-    const int n_part = fused ? fused_grid * fused_pairs(radix) : 0;
     int64_t fused_qc = std::max<int64_t>(
         1, std::min<int64_t>(8192, int64_t(e_bytes / (2 * size_t(M) * cplx))));
     if (const char* cap = std::getenv("RSATB_FFTCHEB_CHUNK")) {  // smaller chunks (tests)
         const int64_t c = std::atoll(cap);
         if (c > 0 && c < fused_qc) fused_qc = c;
     }
-    DevBuf bPart, bTab;
     if (fused) {
-        RSATB_TRY(bPart.alloc(size_t(n_part) * M * sizeof(double2)));
-        RSATB_TRY(bTab.alloc(size_t(M / 4 + M) * sizeof(double2)));
-        fused_tables_kernel<<<(M / 4 + M + 255) / 256, 256, 0, st>>>(M, bWts.as<double>(),
-                                                                     bTab.as<double2>());
+        fused_tables_kernel<<<(M / 4 + M + 255) / 256, 256, 0, st>>>(M, d_wts, d_tab);
         RSATB_LAUNCH_CHECK(ctx);
     }
-
-    // cuFFT plans: full chunks and the last, shorter chunk of a section.
-    Plan plans[2];
-    int64_t plan_nq[2] = {0, 0};
-    auto plan_for = [&](int64_t nq, cufftHandle* out) -> int {
-        for (int i = 0; i < 2; ++i)
-            if (plans[i].made && plan_nq[i] == nq) {
-                *out = plans[i].h;
-                return RSATB_SUCCESS;
-            }
-        int slot_i = plans[0].made ? 1 : 0;
-        if (plans[slot_i].made) {
-            cufftDestroy(plans[slot_i].h);
-            plans[slot_i].made = false;
-        }
-        int n2 = bastin ? 2 * M : M;
-        int emb = n2;
-        RSATB_CUFFT_TRY(cufftPlanMany(&plans[slot_i].h, 1, &n2, &emb, int(nq), 1, &emb, int(nq), 1,
-                                      CUFFT_Z2Z, int(nq)));
-        plans[slot_i].made = true;
-        plan_nq[slot_i] = nq;
-        RSATB_CUFFT_TRY(cufftSetStream(plans[slot_i].h, st));
-        *out = plans[slot_i].h;
-        return RSATB_SUCCESS;
-    };
 
     cudaEvent_t ev0, ev1;
     RSATB_CUDA_TRY(cudaEventCreate(&ev0));
@@ -1291,7 +1364,7 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
         ma.n_rows = N;
         ma.row_ptr = c.op->H->row_ptr;
         ma.col_ind = c.op->H->col_ind;
-        ma.wgt = bWgt.as<T>();
+        ma.wgt = wgt;
         ma.W1 = W1;
         ma.C = moment_threads_per_row<T>(R);
         ma.c = c.op->center;
@@ -1306,11 +1379,11 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
         ma.cap = std::min(kMomentCap, rpc * longest);
         m_smem = size_t(ma.cap) * (4 * sizeof(T) + sizeof(int32_t));
         moment_init_kernel<T><<<grid_for(N * R, ctx->sm_count), 256, 0, st>>>(
-            N, R, ma.row_ptr, ma.col_ind, ma.wgt, psi, ma.cscale, bInit.as<T>());
+            N, R, ma.row_ptr, ma.col_ind, ma.wgt, psi, ma.cscale, start);
         RSATB_LAUNCH_CHECK(ctx);
     } else {
         for (int a = 0; a < 3; ++a)
-            RSATB_TRY(current_rows(c, V[a], W1, psi, J[a], 0, nb, bU.p, bW.p));
+            RSATB_TRY(current_rows(c, V[a], W1, psi, J[a], 0, nb, u_scr, w_scr));
         pack_axes_kernel<T><<<grid_for(N * 3 * R, ctx->sm_count), 256, 0, st>>>(N, R, J[0], J[1],
                                                                                J[2], rinit);
         RSATB_LAUNCH_CHECK(ctx);
@@ -1328,16 +1401,16 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
             // Moment 0 is read from its own buffer, moment 1 formed in panel 0,
             // then the panels alternate (panel 1 takes moment 2 over a copy of
             // moment 0, its predecessor).
-            T* pan[2] = {bPan.as<T>(), bPan.as<T>() + panel};
+            T* pan[2] = {pan0, pan0 + panel};
             if (M > 1)
-                RSATB_CUDA_TRY(cudaMemcpyAsync(pan[1], bInit.p, panel * sizeof(T),
+                RSATB_CUDA_TRY(cudaMemcpyAsync(pan[1], start, panel * sizeof(T),
                                                cudaMemcpyDeviceToDevice, st));
             const int rpc = m_threads / ma.C;
             const unsigned grid = unsigned((N + rpc - 1) / rpc);
             ma.row0 = rows0;
             ma.row1 = rows0 + rows;
             for (int m = 0; m < M; ++m) {
-                ma.cur = m == 0 ? bInit.as<T>() : pan[(m + 1) & 1];
+                ma.cur = m == 0 ? start : pan[(m + 1) & 1];
                 ma.prev = pan[m & 1];
                 ma.sl = SL + 2 * size_t(m) * sslot;
                 ma.sr = SR + 2 * size_t(m) * sslot;
@@ -1373,8 +1446,8 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
                 } else if (m == 1) {
                     T* lo = l[li];
                     li = (li + 1) % 3;
-                    RSATB_TRY(op_step(c, W1, lp, nullptr, lo, bU.p, bW.p, 1.0, 0.0));
-                    RSATB_TRY(op_step(c, W3, r[ri_prev], nullptr, r[1], bU.p, bW.p, 1.0, 0.0));
+                    RSATB_TRY(op_step(c, W1, lp, nullptr, lo, u_scr, w_scr, 1.0, 0.0));
+                    RSATB_TRY(op_step(c, W3, r[ri_prev], nullptr, r[1], u_scr, w_scr, 1.0, 0.0));
                     lc = lo;
                     ri_cur = 1;
                     lm = lc;
@@ -1383,8 +1456,8 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
                     T* lo = l[li];
                     li = (li + 1) % 3;
                     const int rn = 3 - ri_prev - ri_cur;
-                    RSATB_TRY(op_step(c, W1, lc, lp, lo, bU.p, bW.p, 2.0, -1.0));
-                    RSATB_TRY(op_step(c, W3, r[ri_cur], r[ri_prev], r[rn], bU.p, bW.p, 2.0, -1.0));
+                    RSATB_TRY(op_step(c, W1, lc, lp, lo, u_scr, w_scr, 2.0, -1.0));
+                    RSATB_TRY(op_step(c, W3, r[ri_cur], r[ri_prev], r[rn], u_scr, w_scr, 2.0, -1.0));
                     lp = lc;
                     lc = lo;
                     ri_prev = ri_cur;
@@ -1395,7 +1468,7 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
                 T* sl = SL + 2 * size_t(m) * sslot;
                 for (int a = 0; a < 3; ++a)
                     RSATB_TRY(current_rows(c, V[a], W1, lm, sl + 2 * size_t(a) * rows * R, sb0, sb1,
-                                           bU.p, bW.p));
+                                           u_scr, w_scr));
                 if (sizeof(T) == 8 || R % 2 == 0)
                     store_right_vec_kernel<T>
                         <<<grid_for(sslot * 2 * int64_t(sizeof(T)) / 16, ctx->sm_count), 256, 0, st>>>(
@@ -1420,7 +1493,7 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
             T* Tq = reinterpret_cast<T*>(EL);
             for (int a = 0; a < 3; ++a) {
                 RSATB_CUDA_TRY(
-                    cudaMemsetAsync(bPart.p, 0, size_t(n_part) * M * sizeof(double2), st));
+                    cudaMemsetAsync(d_part, 0, size_t(n_part) * M * sizeof(double2), st));
                 for (int64_t i0 = 0; i0 < per_axis; i0 += fused_qc) {
                     const int64_t n = std::min<int64_t>(fused_qc, per_axis - i0);
                     const dim3 gg(unsigned((n + 31) / 32), M / 32, 2);
@@ -1431,27 +1504,37 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
                     if constexpr (std::is_same<T, float>::value) {
                         if (fused32) {
                             RSATB_TRY((fused_launch<T, float2, 8>(ctx, fused_grid, n, Tq,
-                                                                  bTab.as<double2>(),
-                                                                  bPart.as<double2>())));
+                                                                  d_tab,
+                                                                  d_part)));
                             done = true;
                         }
                     }
                     if (!done)
                         RSATB_TRY((fused_launch_r<T, double2>(ctx, radix, fused_grid, n, Tq,
-                                                              bTab.as<double2>(),
-                                                              bPart.as<double2>())));
+                                                              d_tab,
+                                                              d_part)));
                     ++chunks;
                 }
                 fused_reduce_kernel<<<M, 128, 0, st>>>(
-                    M, n_part, bPart.as<double2>(), a == 0 ? 0 : (a == 1 ? 3 : 5), K);
+                    M, n_part, d_part, a == 0 ? 0 : (a == 1 ? 3 : 5), K);
                 RSATB_LAUNCH_CHECK(ctx);
             }
         }
         for (int64_t c0 = 0; !fused && c0 < rows; c0 += chunk_rows) {
             const int64_t cr = std::min<int64_t>(chunk_rows, rows - c0);
             const int64_t nq = 3 * cr * R;
-            cufftHandle plan;
-            RSATB_TRY(plan_for(nq, &plan));
+            cufftHandle plan = 0;
+            size_t wneed = 0;
+            RSATB_TRY(fft_plan(ctx, fft_n, nq, &plan, &wneed));
+            void* area = mem.at<void>(oFft);
+            if (wneed > fft_work) {
+                RSATB_CUDA_TRY(cudaStreamSynchronize(st));
+                extra_work.release();
+                RSATB_TRY(extra_work.alloc(wneed));
+                area = extra_work.p;
+            }
+            RSATB_CUFFT_TRY(cufftSetStream(plan, st));
+            RSATB_CUFFT_TRY(cufftSetWorkArea(plan, area));
             const unsigned gx = std::min(64u, grid_for(nq, ctx->sm_count));
             if (!bastin) {
                 const dim3 grid(gx, M / 2 + 1);
@@ -1459,7 +1542,7 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
                 double2* dst[2] = {EL, ER};
                 for (int t = 0; t < 2; ++t) {
                     dct3_input_kernel<T><<<grid, 256, 0, st>>>(M, nq, int(cr), R, rows, c0, sslot,
-                                                               src[t], bWts.as<double>(), dst[t]);
+                                                               src[t], d_wts, dst[t]);
                     RSATB_LAUNCH_CHECK(ctx);
                     RSATB_CUFFT_TRY(cufftExecZ2Z(plan,
                                                  reinterpret_cast<cufftDoubleComplex*>(dst[t]),
@@ -1470,7 +1553,7 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
                 RSATB_LAUNCH_CHECK(ctx);
             } else {
                 const dim3 grid(gx, M);
-                const double2* w1 = bPw.as<double2>();
+                const double2* w1 = d_pw;
                 const double2* w2 = w1 + M;
                 double2* dst[4] = {EL1, ER1, EL2, ER2};
                 const T* src[4] = {SL, SR, SL, SR};
