@@ -473,7 +473,7 @@ typedef struct {
     double accept;          /* a problem whose final ||X - I||_F exceeds this is reported
                                RSATB_NUMERICAL_FAILURE [1e-6] */
     size_t workspace_bytes; /* device workspace per chunk of problems [8 GiB] */
-    int no_graph;           /* 0: each chunk's iterations run as one captured CUDA graph */
+    int no_graph;           /* accepted and without effect: the iterations are launched directly */
     int tc_kernel;          /* tensor-core GEMM: 0 the built-in choice, 1 warp-specialised
                                (N tile <= 128), 2 single-role (N tile <= 256) */
     int n_tiles;            /* entries of the N-tile table (0: the built-in rule, the fewest

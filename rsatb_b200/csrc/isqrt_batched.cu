@@ -43,6 +43,18 @@ namespace {
 
 // ------------------------------------------------------------ kernels
 
+// f(r, c) for every element of a rows x cols matrix of problem blockIdx.x: rows
+// over the warps of the gridDim.y CTAs that share the problem, columns over the
+// lanes (coalesced, no division).  Several CTAs per problem: with one, a batch
+// of 39 problems took 0.24 ms in each of these kernels.
+template <typename F>
+__device__ __forceinline__ void for_elements(int rows, int cols, F&& f) {
+    const int warps = blockDim.x >> 5;
+    for (int r = blockIdx.y * warps + (threadIdx.x >> 5); r < rows; r += gridDim.y * warps)
+        for (int c = threadIdx.x & 31; c < cols; c += 32) f(r, c);
+}
+
+
 // S (row-major, padded, symmetric from the upper triangle of the
 // column-major input) in FP64 and, for a tensor-core phase, as TF32 hi/lo.
 __global__ void pack_kernel(const Prob* probs, const int64_t* in_off, const double* M,
@@ -50,10 +62,10 @@ __global__ void pack_kernel(const Prob* probs, const int64_t* in_off, const doub
     const Prob pr = probs[blockIdx.x];
     const double* src = M + in_off[blockIdx.x];
     const int np = pr.n_pad, n = pr.n;
-    for (int64_t e = threadIdx.x; e < int64_t(np) * np; e += blockDim.x) {
-        const int r = int(e / np), c = int(e - int64_t(r) * np);
+    for_elements(np, np, [&](int r, int c) {
+        const int e = r * np + c;
         double v = 0.0;
-        if (r < n && c < n) v = (r <= c) ? src[int64_t(c) * n + r] : src[int64_t(r) * n + c];
+        if (r < n && c < n) v = (r <= c) ? src[c * n + r] : src[r * n + c];
         s64[pr.off + e] = v;
         if (s_hi) {
             const float f = float(v);
@@ -61,7 +73,7 @@ __global__ void pack_kernel(const Prob* probs, const int64_t* in_off, const doub
             s_hi[pr.off + e] = h;
             s_lo[pr.off + e] = f - h;
         }
-    }
+    });
 }
 
 // Scale s >= lambda_max, the smaller of two upper bounds, the Gershgorin
@@ -69,18 +81,21 @@ __global__ void pack_kernel(const Prob* probs, const int64_t* in_off, const doub
 // steps: X0 = S / s has its smallest eigenvalue lambda_min / s), and the
 // starting iterate Z0 = I / sqrt(s) in FP64 (and as TF32 hi/lo for a
 // tensor-core phase); state reset.
-__global__ void init_kernel(const Prob* probs, const double* s64, State* st, float* z_hi,
-                            float* z_lo, double* z64, double* scale, int cap) {
+__global__ void init_kernel(const Prob* probs, const double* s64, State* st, double* scale,
+                            int cap) {
     const Prob pr = probs[blockIdx.x];
     const int np = pr.n_pad, n = pr.n;
     __shared__ double red[256], red2[256];
     double m = 0.0, f2 = 0.0;
-    for (int r = threadIdx.x; r < n; r += blockDim.x) {
+    // S is symmetric: column sums, read coalesced.
+    for (int c = threadIdx.x; c < n; c += blockDim.x) {
         double s = 0.0;
-        const double* row = s64 + pr.off + int64_t(r) * np;
-        for (int c = 0; c < n; ++c) {
-            s += fabs(row[c]);
-            f2 += row[c] * row[c];
+        const double* col = s64 + pr.off + c;
+#pragma unroll 8
+        for (int r = 0; r < n; ++r) {
+            const double v = col[r * np];
+            s += fabs(v);
+            f2 += v * v;
         }
         m = fmax(m, s);
     }
@@ -95,18 +110,6 @@ __global__ void init_kernel(const Prob* probs, const double* s64, State* st, flo
         __syncthreads();
     }
     const double s = fmin(red[0], sqrt(red2[0]));
-    const double z0 = s > 0.0 ? 1.0 / sqrt(s) : 0.0;
-    for (int64_t e = threadIdx.x; e < int64_t(np) * np; e += blockDim.x) {
-        const int r = int(e / np), c = int(e - int64_t(r) * np);
-        const double v = (r == c && r < n) ? z0 : 0.0;
-        if (z_hi) {
-            const float f = float(v);
-            const float h = umma::to_tf32(f);
-            z_hi[pr.off + e] = h;
-            z_lo[pr.off + e] = f - h;
-        }
-        z64[pr.off + e] = v;
-    }
     if (threadIdx.x == 0) {
         scale[blockIdx.x] = s;
         State x;
@@ -152,6 +155,27 @@ __global__ void rearm_kernel(int np_count, State* st, int* low_count, int from_l
     st[p] = x;
 }
 
+// Z0 = I / sqrt(s) in FP64 and, for a tensor-core phase, as TF32 hi/lo in Z and
+// in its transpose's first buffer.
+__global__ void start_kernel(const Prob* probs, const double* scale, float* z_hi, float* z_lo,
+                             float* zt_hi, float* zt_lo, double* z64) {
+    const Prob pr = probs[blockIdx.x];
+    const int np = pr.n_pad;
+    const double s = scale[blockIdx.x];
+    const double z0 = s > 0.0 ? 1.0 / sqrt(s) : 0.0;
+    for_elements(np, np, [&](int r, int c) {
+        const int64_t e = pr.off + r * np + c;
+        const double v = (r == c && r < pr.n) ? z0 : 0.0;
+        z64[e] = v;
+        if (z_hi) {
+            const float f = float(v);
+            const float h = umma::to_tf32(f);
+            z_hi[e] = zt_hi[e] = h;
+            z_lo[e] = zt_lo[e] = f - h;
+        }
+    });
+}
+
 // Z64 = I / sqrt(s) for the problems the FP64 phase restarts.
 __global__ void restart_kernel(const Prob* probs, const State* st, const double* scale,
                                double* z64) {
@@ -160,10 +184,9 @@ __global__ void restart_kernel(const Prob* probs, const State* st, const double*
     const int np = pr.n_pad;
     const double s = scale[blockIdx.x];
     const double z0 = s > 0.0 ? 1.0 / sqrt(s) : 0.0;
-    for (int64_t e = threadIdx.x; e < int64_t(np) * np; e += blockDim.x) {
-        const int r = int(e / np), c = int(e - int64_t(r) * np);
-        z64[pr.off + e] = (r == c && r < pr.n) ? z0 : 0.0;
-    }
+    for_elements(np, np, [&](int r, int c) {
+        z64[pr.off + r * np + c] = (r == c && r < pr.n) ? z0 : 0.0;
+    });
 }
 
 // The loop condition of rsatb/calc/isqrtm.hpp:615-640 for every active
@@ -239,8 +262,9 @@ __global__ void retire_low_kernel(const Prob* probs, const State* st, const doub
     if (!st[blockIdx.x].retire) return;
     const Prob pr = probs[blockIdx.x];
     const int np = pr.n_pad;
-    for (int64_t e = threadIdx.x; e < int64_t(np) * np; e += blockDim.x)
-        dst[pr.off + e] = src[pr.off + e];
+    for_elements(np, np, [&](int r, int c) {
+        dst[pr.off + r * np + c] = src[pr.off + r * np + c];
+    });
 }
 
 // z64 = z_hi + z_lo for every problem: the split-TF32 update keeps the
@@ -250,8 +274,10 @@ __global__ void low_to_f64_kernel(const Prob* probs, const float* z_hi, const fl
                                   double* z64) {
     const Prob pr = probs[blockIdx.x];
     const int np = pr.n_pad;
-    for (int64_t e = threadIdx.x; e < int64_t(np) * np; e += blockDim.x)
-        z64[pr.off + e] = double(z_hi[pr.off + e]) + double(z_lo[pr.off + e]);
+    for_elements(np, np, [&](int r, int c) {
+        const int64_t e = pr.off + r * np + c;
+        z64[e] = double(z_hi[e]) + double(z_lo[e]);
+    });
 }
 
 // Result of a problem the FP64 phase just stopped: columns
@@ -263,11 +289,10 @@ __global__ void retire_out_kernel(const Prob* probs, const State* st, const doub
     const Prob pr = probs[blockIdx.x];
     const int np = pr.n_pad, n = pr.n, c0 = col_start[blockIdx.x], k = k_cols[blockIdx.x];
     double* dst = out + out_off[blockIdx.x];
-    for (int64_t e = threadIdx.x; e < int64_t(n) * k; e += blockDim.x) {
-        const int j = int(e / n), i = int(e - int64_t(j) * n);
+    for_elements(k, n, [&](int j, int i) {
         const int c = c0 + j;
-        dst[e] = 0.5 * (z64[pr.off + int64_t(i) * np + c] + z64[pr.off + int64_t(c) * np + i]);
-    }
+        dst[int64_t(j) * n + i] = 0.5 * (z64[pr.off + i * np + c] + z64[pr.off + c * np + i]);
+    });
 }
 
 struct F64Item {
@@ -537,7 +562,6 @@ struct Opts {
     double tol;
     double accept;
     size_t workspace;
-    bool graph;
     bool ws;                                // warp-specialised tensor-core kernel
     std::vector<std::pair<int, int>> tiles; // (n_pad, N tile) overrides
 };
@@ -641,35 +665,42 @@ int f64_gemm(rsatb_context* ctx, const Dev& d, const double* A, const double* B,
     return RSATB_SUCCESS;
 }
 
-// Issues `body` either directly or as one captured graph on the context's
-// stream.
+// Issues body(k, last) for k = 0 .. n and stops after an iteration that left no
+// problem going (live[k], set by its control step).  The flag is read back one
+// iteration behind, so the device always has the next iteration queued and at
+// most one iteration of no-ops runs at the end.  (As one captured graph of all
+// n iterations, capture and instantiation came before the first kernel and the
+// empty iterations after the last live one: 1.2 ms of a 4.5 ms batch of 39.)
 template <typename F>
-int run_phase(rsatb_context* ctx, bool graph, F&& body) {
-    if (!graph || ctx->stream == nullptr) return body();
-    RSATB_CUDA_TRY(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-    const int st = body();
-    cudaGraph_t g = nullptr;
-    const cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
-    if (st != RSATB_SUCCESS) {
-        if (g) cudaGraphDestroy(g);
-        return st;
+int run_phase(rsatb_context* ctx, int n, const int* live, F&& body) {
+    void* pin = nullptr;
+    RSATB_TRY(ctx_pinned(ctx, (size_t(n) + 1) * sizeof(int), &pin));
+    volatile int* flag = static_cast<volatile int*>(pin);
+    struct Events {
+        cudaEvent_t e[2] = {nullptr, nullptr};
+        ~Events() {
+            for (auto x : e)
+                if (x) cudaEventDestroy(x);
+        }
+    } ev;
+    for (auto& x : ev.e) RSATB_CUDA_TRY(cudaEventCreateWithFlags(&x, cudaEventDisableTiming));
+    for (int k = 0; k <= n; ++k) {
+        RSATB_TRY(body(k, k == n));
+        if (k == n) break;
+        RSATB_CUDA_TRY(cudaMemcpyAsync(const_cast<int*>(flag) + k, live + k, sizeof(int),
+                                       cudaMemcpyDeviceToHost, ctx->stream));
+        RSATB_CUDA_TRY(cudaEventRecord(ev.e[k & 1], ctx->stream));
+        if (k == 0) continue;
+        RSATB_CUDA_TRY(cudaEventSynchronize(ev.e[(k - 1) & 1]));
+        if (flag[k - 1] == 0) break;
     }
-    if (e != cudaSuccess)
-        return set_error(RSATB_CUDA_ERROR, "graph capture failed: %s", cudaGetErrorString(e));
-    cudaGraphExec_t x = nullptr;
-    cudaError_t ie = cudaGraphInstantiate(&x, g, 0);
-    cudaGraphDestroy(g);
-    if (ie != cudaSuccess)
-        return set_error(RSATB_CUDA_ERROR, "graph instantiation failed: %s",
-                         cudaGetErrorString(ie));
-    const cudaError_t le = cudaGraphLaunch(x, ctx->stream);
-    const cudaError_t se = cudaStreamSynchronize(ctx->stream);
-    cudaGraphExecDestroy(x);
-    if (le != cudaSuccess)
-        return set_error(RSATB_CUDA_ERROR, "graph launch failed: %s", cudaGetErrorString(le));
-    if (se != cudaSuccess)
-        return set_error(RSATB_CUDA_ERROR, "graph run failed: %s", cudaGetErrorString(se));
     return RSATB_SUCCESS;
+}
+
+// CTAs per problem of the element-wise kernels: about eight per SM in all.
+dim3 element_grid(const rsatb_context* ctx, int P) {
+    const int y = (ctx->sm_count * 8 + P - 1) / P;
+    return dim3(unsigned(P), unsigned(y < 1 ? 1 : y > 32 ? 32 : y));
 }
 
 int run_chunk(rsatb_context* ctx, const Opts& o, const Chunk& ch, const int* col_start_h,
@@ -818,17 +849,16 @@ int run_chunk(rsatb_context* ctx, const Opts& o, const Chunk& ch, const int* col
     RSATB_CUDA_TRY(cudaMemsetAsync(d.live, 0, size_t(d.n_live) * sizeof(int), s));
 
     // Pack S and the starting iterate.
-    pack_kernel<<<P, 256, 0, s>>>(d.probs, d.in_off, M, a.s64, a.s_hi, a.s_lo);
+    const dim3 eg = element_grid(ctx, P);
+    pack_kernel<<<eg, 256, 0, s>>>(d.probs, d.in_off, M, a.s64, a.s_hi, a.s_lo);
     RSATB_LAUNCH_CHECK(ctx);
-    init_kernel<<<P, 256, 0, s>>>(d.probs, a.s64, d.state, a.z_hi, a.z_lo, a.z64[0], d.scale,
+    init_kernel<<<P, 256, 0, s>>>(d.probs, a.s64, d.state, d.scale,
                                   low ? o.max_iter : o.max_fp64);
     RSATB_LAUNCH_CHECK(ctx);
-    if (low) {  // Z0 = I / sqrt(s) is symmetric: Z0^T = Z0
-        RSATB_CUDA_TRY(cudaMemcpyAsync(a.zt_hi[0], a.z_hi, E * sizeof(float),
-                                       cudaMemcpyDeviceToDevice, s));
-        RSATB_CUDA_TRY(cudaMemcpyAsync(a.zt_lo[0], a.z_lo, E * sizeof(float),
-                                       cudaMemcpyDeviceToDevice, s));
-    }
+    // Z0 is symmetric: Z0^T = Z0
+    start_kernel<<<eg, 256, 0, s>>>(d.probs, d.scale, low ? a.z_hi : nullptr, a.z_lo, a.zt_hi[0],
+                                    a.zt_lo[0], a.z64[0]);
+    RSATB_LAUNCH_CHECK(ctx);
     const int cb = (P + 255) / 256;
 
     cudaEvent_t ev[3];
@@ -849,28 +879,31 @@ int run_chunk(rsatb_context* ctx, const Opts& o, const Chunk& ch, const int* col
     const int floor_stop = floor_stop_enabled() ? 1 : 0;
     if (low) {
         RSATB_TRY(prepare_tc_gemm());
-        RSATB_TRY(run_phase(ctx, o.graph, [&]() -> int {
-            for (int k = 0; k <= o.max_iter; ++k) {
+        RSATB_TRY(run_phase(ctx, o.max_iter, d.live, [&](int k, bool last) -> int {
+            {
                 const int c = k & 1;
                 const int* live_in = k ? d.live + (k - 1) : nullptr;  // after control k - 1
                 const int* live_k = d.live + k;                        // after control k
-                // W = Z S^T, X = Z W^T (+ residual) on the tensor cores
-                RSATB_TRY(tc_gemm(ctx, ch, d, d.tc_items, group_begin, a.z_hi, a.z_lo, a.s_hi,
-                                  a.s_lo, a.w_hi, a.w_lo, nullptr, EPI_STORE, nullptr, nullptr,
-                                  split, o.ws, stats, nullptr, nullptr, false, live_in));
+                // W = Z S^T, X = Z W^T (+ residual) on the tensor cores, each formed
+                // as its transpose (S Z^T, W Z^T) and stored transposed: for a
+                // fixed column a warp's 32 rows are one coalesced line, where the
+                // direct store touches a line per row.
+                RSATB_TRY(tc_gemm(ctx, ch, d, d.tc_items, group_begin, a.s_hi, a.s_lo, a.z_hi,
+                                  a.z_lo, nullptr, nullptr, nullptr, EPI_STORE, nullptr, nullptr,
+                                  split, o.ws, stats, a.w_hi, a.w_lo, false, live_in));
                 // X on every tile (its upper triangle mirrored, as P is, measured
                 // the same: 21,300 against 21,400 matrices/s at 20,000 problems).
-                RSATB_TRY(tc_gemm(ctx, ch, d, d.tc_items, group_begin, a.z_hi, a.z_lo, a.w_hi,
-                                  a.w_lo, a.x_hi, a.x_lo, nullptr, EPI_RESID, nullptr, nullptr,
-                                  split, o.ws, stats, nullptr, nullptr, false, live_in));
+                RSATB_TRY(tc_gemm(ctx, ch, d, d.tc_items, group_begin, a.w_hi, a.w_lo, a.z_hi,
+                                  a.z_lo, nullptr, nullptr, nullptr, EPI_RESID, nullptr, nullptr,
+                                  split, o.ws, stats, a.x_hi, a.x_lo, false, live_in));
                 control_kernel<<<cb, 256, 0, s>>>(P, d.state, d.res2, o.tol, 1, lift,
                                                   floor_stop, d.live + k);
                 RSATB_LAUNCH_CHECK(ctx);
                 if (c == 1 && update64) {
-                    retire_low_kernel<<<P, 256, 0, s>>>(d.probs, d.state, a.z64[1], a.z64[0]);
+                    retire_low_kernel<<<eg, 256, 0, s>>>(d.probs, d.state, a.z64[1], a.z64[0]);
                     RSATB_LAUNCH_CHECK(ctx);
                 }
-                if (k == o.max_iter) break;
+                if (last) return RSATB_SUCCESS;
                 // P = 1.875 I - 1.25 X + 0.375 X X^T (or the lift polynomial) on
                 // the tensor cores, then
                 // Z' = P Z with P exactly symmetric.  A symmetric factor on the
@@ -908,7 +941,7 @@ int run_chunk(rsatb_context* ctx, const Opts& o, const Chunk& ch, const int* col
         }));
     }
     if (low && !update64) {
-        low_to_f64_kernel<<<P, 256, 0, s>>>(d.probs, a.z_hi, a.z_lo, a.z64[0]);
+        low_to_f64_kernel<<<eg, 256, 0, s>>>(d.probs, a.z_hi, a.z_lo, a.z64[0]);
         RSATB_LAUNCH_CHECK(ctx);
     }
     RSATB_CUDA_TRY(cudaEventRecord(ev[1], s));
@@ -916,9 +949,9 @@ int run_chunk(rsatb_context* ctx, const Opts& o, const Chunk& ch, const int* col
     rearm_kernel<<<cb, 256, 0, s>>>(P, d.state, d.low_count, low ? 1 : 0, o.max_fp64,
                                     o.max_fp64_restart, kRestartAbove);
     RSATB_LAUNCH_CHECK(ctx);
-    restart_kernel<<<P, 256, 0, s>>>(d.probs, d.state, d.scale, a.z64[0]);
+    restart_kernel<<<eg, 256, 0, s>>>(d.probs, d.state, d.scale, a.z64[0]);
     RSATB_LAUNCH_CHECK(ctx);
-    retire_out_kernel<<<P, 256, 0, s>>>(d.probs, d.state, a.z64[0], d.col_start, d.k_cols,
+    retire_out_kernel<<<eg, 256, 0, s>>>(d.probs, d.state, a.z64[0], d.col_start, d.k_cols,
                                         d.out_off, out);
     RSATB_LAUNCH_CHECK(ctx);
     int fp64_steps = o.max_fp64;
@@ -933,8 +966,8 @@ int run_chunk(rsatb_context* ctx, const Opts& o, const Chunk& ch, const int* col
             if (x.active && x.cap > fp64_steps) fp64_steps = x.cap;
     }
 
-    RSATB_TRY(run_phase(ctx, o.graph, [&]() -> int {
-        for (int k = 0; k <= fp64_steps; ++k) {
+    RSATB_TRY(run_phase(ctx, fp64_steps, d.live_f64, [&](int k, bool last) -> int {
+        {
             const int c = k & 1;
             const int* live_in = k ? d.live_f64 + (k - 1) : nullptr;
             const int* live_k = d.live_f64 + k;
@@ -945,10 +978,10 @@ int run_chunk(rsatb_context* ctx, const Opts& o, const Chunk& ch, const int* col
             control_kernel<<<cb, 256, 0, s>>>(P, d.state, d.res2, o.tol, 0, 0, 0,
                                               d.live_f64 + k);
             RSATB_LAUNCH_CHECK(ctx);
-            retire_out_kernel<<<P, 256, 0, s>>>(d.probs, d.state, a.z64[c], d.col_start,
+            retire_out_kernel<<<eg, 256, 0, s>>>(d.probs, d.state, a.z64[c], d.col_start,
                                                 d.k_cols, d.out_off, out);
             RSATB_LAUNCH_CHECK(ctx);
-            if (k == fp64_steps) break;
+            if (last) return RSATB_SUCCESS;
             // X and P exactly symmetric (upper tiles, mirrored): Z' = P Z
             // takes P as it is.
             RSATB_TRY(f64_gemm<true>(ctx, d, a.x64, a.x64, a.p64, EPI_POLY, a.x64, stats,
@@ -1040,7 +1073,6 @@ extern "C" int rsatb_isqrt_columns_batched(rsatb_ctx_t ctx, int n_problems, cons
     o.accept = (options && options->accept > 0) ? options->accept : 1e-6;
     o.workspace = (options && options->workspace_bytes) ? options->workspace_bytes
                                                         : (size_t(8) << 30);
-    o.graph = !(options && options->no_graph);
     const int tck = options ? options->tc_kernel : 0;
     if (tck < 0 || tck > 2) return set_error(RSATB_INVALID_ARGUMENT, "unknown tc_kernel %d", tck);
     o.ws = tck == 0 ? default_tc_ws() : tck == 1;
@@ -1072,25 +1104,6 @@ extern "C" int rsatb_isqrt_columns_batched(rsatb_ctx_t ctx, int n_problems, cons
     }
     if (!(reinterpret_cast<uintptr_t>(M) % 8 == 0) || !(reinterpret_cast<uintptr_t>(out) % 8 == 0))
         return set_error(RSATB_INVALID_ARGUMENT, "M and out must be 8-byte aligned");
-
-    // Graph capture needs a capturable stream: on the legacy default stream
-    // the call runs on the context's own stream, ordered after the work
-    // already queued on the caller's.
-    struct StreamSwap {
-        rsatb_context* ctx;
-        cudaStream_t saved;
-        ~StreamSwap() { ctx->stream = saved; }
-    } swap{ctx, ctx->stream};
-    if (o.graph && ctx->stream == nullptr && ctx->own_stream != nullptr) {
-        cudaEvent_t e;
-        RSATB_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        cudaError_t r1 = cudaEventRecord(e, nullptr);
-        cudaError_t r2 = cudaStreamWaitEvent(ctx->own_stream, e, 0);
-        cudaEventDestroy(e);
-        RSATB_CUDA_TRY(r1);
-        RSATB_CUDA_TRY(r2);
-        ctx->stream = ctx->own_stream;
-    }
 
     // Largest first, so each chunk's buckets are ordered and the persistent
     // CTAs start on the longest tiles.
