@@ -42,20 +42,53 @@ __device__ __forceinline__ void record_error(unsigned* error, unsigned code) {
 // args.sym only the upper triangle (col >= row) is stored, each element
 // also at (col, row), so C leaves exactly symmetric.  The transposed and
 // mirrored stores of a warp (32 consecutive rows, one column) are
-// coalesced.
-// X (hi + lo) at 16 consecutive elements for the polynomial epilogue, as
-// 128-bit loads.
-__device__ __forceinline__ void load_x16(const TcArgs& args, int64_t base, float (&xe)[16]) {
-    const float4* h = reinterpret_cast<const float4*>(args.xe_hi + base);
-    const float4* l = reinterpret_cast<const float4*>(args.xe_lo + base);
+// coalesced; a warp's rows are a whole 32 of the padded problem, so the row
+// stores are formed by the warp together (store_rows_warp).
+// X (hi + lo) at (row, col0 .. col0 + 15) for the polynomial epilogue, read as
+// (col, row): X is symmetric up to rounding, and for a fixed column a warp's 32
+// rows are one 128-byte line (16 bytes a row, 32 lines an instruction, the other
+// way).
+__device__ __forceinline__ void load_x16(const TcArgs& args, const Prob& pr, int row, int col0,
+                                         float (&xe)[16]) {
+    const int64_t base = pr.off + int64_t(col0) * pr.n_pad + row;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const float4 a = h[q], b = l[q];
-        xe[4 * q] = a.x + b.x;
-        xe[4 * q + 1] = a.y + b.y;
-        xe[4 * q + 2] = a.z + b.z;
-        xe[4 * q + 3] = a.w + b.w;
+    for (int j = 0; j < 16; ++j)
+        xe[j] = args.xe_hi[base + j * pr.n_pad] + args.xe_lo[base + j * pr.n_pad];
+}
+
+// 4 x 4 transpose of 16-byte quads over groups of four lanes: in, lane i holds
+// quads 0..3 of its row; out, quad i of the group's rows 0..3.
+__device__ __forceinline__ void quad_transpose(float (&v)[16], int lane) {
+#pragma unroll
+    for (int s = 1; s <= 2; s <<= 1) {
+        const bool up = lane & s;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (q & s) continue;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                float& x = v[4 * q + e];
+                float& y = v[4 * (q + s) + e];
+                const float got = __shfl_xor_sync(0xffffffffu, up ? x : y, s);
+                if (up) x = got;
+                else y = got;
+            }
+        }
     }
+}
+
+// The 16 consecutive columns of a warp's 32 rows (row: this lane's), 64
+// contiguous bytes of a row per four lanes: 8 lines an instruction where 16
+// bytes per lane touch 32.
+__device__ __forceinline__ void store_rows_warp(float* c, const Prob& pr, int row, int col0,
+                                                float (&v)[16]) {
+    const int lane = threadIdx.x & 31;
+    quad_transpose(v, lane);
+    float* p = c + pr.off + int64_t(row - (lane & 3)) * pr.n_pad + col0 + 4 * (lane & 3);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        *reinterpret_cast<float4*>(p + int64_t(j) * pr.n_pad) =
+            make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
 }
 
 __device__ __forceinline__ void store_rows(const TcArgs& args, int64_t base,
@@ -79,13 +112,18 @@ __device__ __forceinline__ void store_rows(const TcArgs& args, int64_t base,
 }
 
 __device__ __forceinline__ void store_chunk(const TcArgs& args, const Prob& pr, int row, int col0,
-                                            const float (&hi)[16], const float (&lo)[16]) {
+                                            float (&hi)[16], float (&lo)[16]) {
     const int np = pr.n_pad;
     const int64_t base = pr.off + int64_t(row) * np + col0;
     if (args.sym) {
-        if (col0 + 15 < row) return;  // below the diagonal: the mirror of another thread's
-        if (col0 >= row) {
-            store_rows(args, base, hi, lo);  // the whole chunk is on or above the diagonal
+        const int row0 = row - (threadIdx.x & 31);  // the warp's first row
+        if (col0 + 15 < row0) return;  // below the diagonal: the mirror of another thread's
+        const bool whole = col0 >= row0 + 31;  // every row's chunk on or above the diagonal
+        if (whole) {
+        } else if (col0 + 15 < row) {
+            return;
+        } else if (col0 >= row) {
+            store_rows(args, base, hi, lo);
         } else {
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
@@ -104,9 +142,16 @@ __device__ __forceinline__ void store_chunk(const TcArgs& args, const Prob& pr, 
             args.c_lo[t] = lo[j];
             if (args.c64) args.c64[t] = double(hi[j]) + double(lo[j]);
         }
+        if (whole) {
+            if (args.c64) {
+                store_rows(args, base, hi, lo);
+            } else {
+                store_rows_warp(args.c_hi, pr, row, col0, hi);
+                store_rows_warp(args.c_lo, pr, row, col0, lo);
+            }
+        }
         return;
     }
-    store_rows(args, base, hi, lo);
     if (args.ct_hi) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
@@ -114,6 +159,12 @@ __device__ __forceinline__ void store_chunk(const TcArgs& args, const Prob& pr, 
             args.ct_hi[t] = hi[j];
             args.ct_lo[t] = lo[j];
         }
+    }
+    if (args.c64) {
+        store_rows(args, base, hi, lo);
+    } else if (args.c_hi) {
+        store_rows_warp(args.c_hi, pr, row, col0, hi);
+        store_rows_warp(args.c_lo, pr, row, col0, lo);
     }
 }
 
@@ -242,7 +293,7 @@ __global__ void __launch_bounds__(128, 1)
                 if (!in_mat || col0 >= np) continue;
                 const int64_t base = pr.off + int64_t(row) * np + col0;
                 float hi[16], lo[16], xe[16];
-                if (args.mode == EPI_POLY) load_x16(args, base, xe);
+                if (args.mode == EPI_POLY) load_x16(args, pr, row, col0, xe);
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
                     const int col = col0 + j;
@@ -318,7 +369,7 @@ __device__ __forceinline__ void ws_epilogue(const TcArgs& args, const TcItem& it
         if (in_mat && col0 < np) {
             const int64_t base = pr.off + int64_t(row) * np + col0;
             float hi[16], lo[16], xe[16];
-            if (args.mode == EPI_POLY) load_x16(args, base, xe);
+            if (args.mode == EPI_POLY) load_x16(args, pr, row, col0, xe);
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
                 const int col = col0 + j;
