@@ -1,0 +1,12 @@
+// Launches and FP64 instantiations of the any-shape tensor-core step.
+#include "cheb_dmma_any_launch.cuh"
+
+namespace rsatb_b200 {
+namespace step_detail {
+
+template int launch_dmma_any<double, false, false>(rsatb_context*, StepArgs&);
+template int launch_dmma_any<double, false, true>(rsatb_context*, StepArgs&);
+template int launch_dmma_any<double, true, true>(rsatb_context*, StepArgs&);
+
+}  // namespace step_detail
+}  // namespace rsatb_b200

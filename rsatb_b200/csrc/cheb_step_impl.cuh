@@ -9,35 +9,12 @@
 #include "cheb_narrow.cuh"
 #include "cheb_dmma.cuh"
 #include "cheb_tf32.cuh"
+#include "step_launch.cuh"
 
 #include <cstdlib>
-#include <mutex>
-#include <unordered_map>
 
 namespace rsatb_b200 {
 namespace step_detail {
-
-// Resident CTAs per SM for a kernel at a given CTA size and shared memory.
-inline int occupancy(const void* kernel, int threads, size_t smem) {
-    static std::mutex mu;
-    static std::unordered_map<uint64_t, int> cache;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const uint64_t key = (uint64_t(reinterpret_cast<uintptr_t>(kernel)) << 8) ^
-                         (uint64_t(threads) << 40) ^ (uint64_t(smem) << 20) ^ uint64_t(dev);
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        auto it = cache.find(key);
-        if (it != cache.end()) return it->second;
-    }
-    int n = 1;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem) != cudaSuccess ||
-        n < 1)
-        n = 1;
-    std::lock_guard<std::mutex> lock(mu);
-    cache[key] = n;
-    return n;
-}
 
 // Optional tuning override of the values-per-thread choice (RSATB_STEP_V).
 inline int env_v() {
@@ -96,8 +73,6 @@ inline int pick_v(int W, bool cv, bool any_b, int block_size, bool dbl) {
     return 0;
 }
 
-constexpr int kNotApplicable = 1000;
-
 // RSATB_STEP_KERNEL=v1|staged|rowsplit|bulk|narrow|dmma|tf32|generic forces one kernel family
 // (tuning and A/B tests); unset picks by shape and precision.
 inline int env_kernel() {
@@ -108,6 +83,7 @@ inline int env_kernel() {
     if (s[0] == 'r') return 3;
     if (s[0] == 'b') return 4;
     if (s[0] == 'n') return 5;
+    if (s[0] == 'd' && s[1] == 'm' && s[2] == 'm' && s[3] == 'a' && s[4] == '_') return 9;  // dmma_any
     if (s[0] == 'd') return 6;
     if (s[0] == 't') return 7;
     if (s[0] == 'g') return 8;  // the register kernel
@@ -512,6 +488,28 @@ int launch_b(rsatb_context* ctx, int V, int64_t rows, StepArgs& a) {
     return set_error(RSATB_NOT_SUPPORTED, "no step kernel for V=%d", V);
 }
 
+// Where the any-shape tensor-core kernel is the default, measured on 4,096 block
+// rows of 17 blocks of 5 and 29 blocks of 8 (us per step of the doubled
+// recurrence, or per Y = A X where marked *; it against the best of the others).
+// W = 8, 16, 32, 64, 128 and 256 on blocks of 8 in FP64 (W <= 16 in FP32) stay
+// with the tiled tensor-core kernel before it, equal or faster.
+//   FP64 b = 8     every width: 7* 13 / 66, 24* 25 / 68, 45 78 / 218, 57* 67 / 188
+//   FP64 b < 8     b = 5: 8 18 / 34, 16 25 / 26, 24* 16 / 24, 45* 31 / 39, 57*
+//                  35 / 43; behind at multiples of 4 from 32 (33 / 30, 64 59 / 38)
+//   FP64 complex   b = 5, 6 columns 28 / 37, 16 35 / 34, 24 45 / 53; 32* 43 / 40,
+//                  64* 76 / 70, but 45* 60 / 62 and 57* 76 / 88, where the others
+//                  lose their wide loads
+//   FP32 b = 8     W < 64 off the bulk-copy widths: 7 20 / 38, 24 32 / 40, 45 60 /
+//                  81; complex panels of W = 90* 73 / 62
+//   FP32 b < 8     W <= 24: 7* 8.6 / 13.5, 16* 11 / 17, 24* 15 / 17; 32* 16 / 15
+//   FP32 complex   W <= 16: 6 columns 24 / 32, 8 24 / 31; 11* 29 / 21
+inline bool dmma_any_wanted(int W, int b, bool cm, bool dbl) {
+    if (dbl) return cm ? W <= 48 || W % 8 != 0 : b == 8 || W < 32 || W % 4 != 0;
+    if (cm) return W <= 16;
+    if (b != 8) return W <= 24;
+    return W < 64 && W != 32;
+}
+
 template <typename VT, typename MT, bool CM, bool CV>
 int launch_typed(rsatb_context* ctx, int block_size, StepArgs& a) {
     const bool special = block_size == 1 || block_size == 5 || block_size == 8;
@@ -539,6 +537,10 @@ int launch_typed(rsatb_context* ctx, int block_size, StepArgs& a) {
             if (st != kNotApplicable) return st;
         }
     }
+    if (forced == 9 || (forced == 0 && dmma_any_wanted(a.W, block_size, CM, sizeof(VT) == 8))) {
+        const int st = launch_dmma_any<VT, CM, CV>(ctx, a);
+        if (st != kNotApplicable) return st;
+    }
     if constexpr (!CM) {
         // Narrow-panel lock-step kernel: blocks of 8, W <= 16 (when forced).
         if (block_size == 8 && forced == 5) {
@@ -555,8 +557,11 @@ int launch_typed(rsatb_context* ctx, int block_size, StepArgs& a) {
     }
     if constexpr (sizeof(VT) == 4 && !CM) {
         // Bulk-copy kernel: FP32, blocks of 8, panels of 32 to 256 values
-        // by default (every width when forced).
-        const bool wide = a.W >= 32;
+        // by default (every width when forced), where its CTAs of 1024 / W
+        // block rows are two per SM or more (4,096 rows, Y = A X: W = 32 39 us
+        // against the register kernel's 25, W = 64 43 against 37; 32,768 rows,
+        // W = 32 152 us).
+        const bool wide = a.W >= 32 && a.n_block_rows * a.W >= int64_t(296) * 1024;
         if (block_size == 8 && (forced == 4 || (forced == 0 && wide))) {
             const int st = launch_bulk<CV>(ctx, a);
             if (st != kNotApplicable) return st;
