@@ -50,15 +50,19 @@ __device__ __forceinline__ double2 col_value(const double* d, int c) {
 // a converged column, |rr_c| < tol2, or a broken-down one, |pap_c| < 1e-14
 // |rr_c|), and rr_out_c = <R_c|R_c> of the updated R: thread (sub, column)
 // of a CTA walks every (subs x gridDim.x)-th row, the CTA sums its rows in
-// a fixed order, and the last CTA to finish (ticket counter) sums the CTA
-// partials in a fixed order and resets the counter.  Deterministic.
+// a fixed order, and the CTA partials are summed as finish_partials sums them,
+// in two levels of 32 CTAs (kGroupCounter0).  Deterministic.  The last CTA also
+// writes the residuals to host memory (pinned), which the host reads after the
+// event behind this launch: no copy between the iterations.
+// 32,768 rows x 16 FP64 columns: 10.6 us with four CTAs per SM (eight 13.9; two
+// and one level 11.8, with a 2.9 us copy behind it).
 template <typename T, bool CV>
 __global__ void __launch_bounds__(kDotThreads)
 cg_update_kernel(T* __restrict__ X, const T* __restrict__ P, T* __restrict__ R,
                  const T* __restrict__ AP, const double* __restrict__ rr,
                  const double* __restrict__ pap, double tol2, int64_t n_rows, int ncols,
-                 double* __restrict__ part, double* __restrict__ rr_out,
-                 unsigned* __restrict__ counter) {
+                 double* part, double* __restrict__ rr_out, double* rr_host,
+                 unsigned* counter) {
     __shared__ double red[kDotThreads];
     __shared__ unsigned ticket;
     const int subs = kDotThreads / ncols;
@@ -105,31 +109,38 @@ cg_update_kernel(T* __restrict__ X, const T* __restrict__ P, T* __restrict__ R,
     }
     __threadfence();
     __syncthreads();
+    int n = int(gridDim.x);
+    size_t step = ncols;
+    const int groups = (n + kGroupCtas - 1) / kGroupCtas;
+    if (groups > 1 && groups <= kMaxGroups) {
+        const int group = blockIdx.x / kGroupCtas;
+        const int size = min(kGroupCtas, n - group * kGroupCtas);
+        unsigned* gc = counter + kGroupCounter0 + group;
+        if (threadIdx.x == 0) ticket = atomicAdd(gc, 1u);
+        __syncthreads();
+        if (ticket != unsigned(size - 1)) return;
+        __threadfence();
+        if (threadIdx.x == 0) *gc = 0u;
+        double* mine = part + size_t(group) * kGroupCtas * ncols;
+        sum_partials(mine, size, ncols, ncols, mine);
+        n = groups;
+        step = size_t(kGroupCtas) * ncols;
+        __threadfence();
+        __syncthreads();
+    }
     if (threadIdx.x == 0) ticket = atomicAdd(counter, 1u);
     __syncthreads();
-    if (ticket != gridDim.x - 1) return;
+    if (ticket != unsigned(n - 1)) return;
     __threadfence();
-    // Eight independent partial sums per thread, so eight L2 loads are in
-    // flight at once (a single chain costs one L2 round trip per CTA).
-    double t8[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    if (sub < subs) {
-        unsigned g = sub;
-        for (; g + 7 * subs < gridDim.x; g += 8 * subs) {
-#pragma unroll
-            for (int u = 0; u < 8; ++u) t8[u] += __ldcg(part + int64_t(g + u * subs) * ncols + col);
-        }
-        for (; g < gridDim.x; g += subs) t8[0] += __ldcg(part + int64_t(g) * ncols + col);
-    }
-    red[threadIdx.x] = ((t8[0] + t8[1]) + (t8[2] + t8[3])) + ((t8[4] + t8[5]) + (t8[6] + t8[7]));
+    sum_partials(part, n, step, ncols, red);
     __syncthreads();
     if (threadIdx.x < ncols) {
-        double u = 0.0;
-        for (int q = 0; q < subs; ++q) u += red[q * ncols + threadIdx.x];
+        const double u = red[threadIdx.x];
         if constexpr (CV) {
-            rr_out[2 * threadIdx.x] = u;
-            rr_out[2 * threadIdx.x + 1] = 0.0;
+            rr_out[2 * threadIdx.x] = rr_host[2 * threadIdx.x] = u;
+            rr_out[2 * threadIdx.x + 1] = rr_host[2 * threadIdx.x + 1] = 0.0;
         } else {
-            rr_out[threadIdx.x] = u;
+            rr_out[threadIdx.x] = rr_host[threadIdx.x] = u;
         }
     }
     if (threadIdx.x == 0) *counter = 0u;  // ready for the next launch
@@ -263,11 +274,11 @@ int axpby(const SolveCall& s, double a, const void* X, double b, void* Y) {
 
 template <typename T, bool CV>
 int update_t(const SolveCall& s, const SolveWork& w, void* X, const double* rr, double tol2,
-             double* rr_out) {
+             double* rr_out, double* rr_host) {
     cg_update_kernel<T, CV><<<w.grid, kDotThreads, 0, s.ctx->stream>>>(
         static_cast<T*>(X), static_cast<const T*>(w.P), static_cast<T*>(w.R),
         static_cast<const T*>(w.AP), rr, w.d_pap, tol2, s.n_rows, s.ncols, w.part, rr_out,
-        w.counter);
+        rr_host, w.counter);
     RSATB_LAUNCH_CHECK(s.ctx);
     return RSATB_SUCCESS;
 }
@@ -283,13 +294,13 @@ int direction_t(const SolveCall& s, const SolveWork& w, const double* rr_old,
 }
 
 int update(const SolveCall& s, const SolveWork& w, void* X, const double* rr, double tol2,
-           double* rr_out) {
+           double* rr_out, double* rr_host) {
     const bool cv = dtype_is_complex(s.vdt);
     if (dtype_is_double(s.vdt))
-        return cv ? update_t<double, true>(s, w, X, rr, tol2, rr_out)
-                  : update_t<double, false>(s, w, X, rr, tol2, rr_out);
-    return cv ? update_t<float, true>(s, w, X, rr, tol2, rr_out)
-              : update_t<float, false>(s, w, X, rr, tol2, rr_out);
+        return cv ? update_t<double, true>(s, w, X, rr, tol2, rr_out, rr_host)
+                  : update_t<double, false>(s, w, X, rr, tol2, rr_out, rr_host);
+    return cv ? update_t<float, true>(s, w, X, rr, tol2, rr_out, rr_host)
+              : update_t<float, false>(s, w, X, rr, tol2, rr_out, rr_host);
 }
 
 int direction(const SolveCall& s, const SolveWork& w, const double* o, const double* n) {
@@ -351,7 +362,7 @@ int cg_core(const SolveCall& s, const SolveWork& w, const rsatb_bsr_matrix* S,
     double* rr = w.d_rr;
     double* rr_new = w.d_rr2;
     RSATB_TRY(dots(s, w, w.R, w.R, rr));
-    // The column residuals of iteration k are copied to pinned memory and
+    // The column residuals of iteration k are written to pinned memory and
     // read after iteration k + 1 has been queued, so the device never waits
     // for the host's test.  A column whose residual is below tol is frozen
     // by the alpha kernel (alpha = 0: X and R unchanged), so once every
@@ -390,9 +401,7 @@ int cg_core(const SolveCall& s, const SolveWork& w, const rsatb_bsr_matrix* S,
     };
     for (int k = 0; k < max_iter && !done; ++k) {
         RSATB_TRY(apply_A(s, w, S, Z, ZH, w.P, w.AP, w.d_pap));
-        RSATB_TRY(update(s, w, X, rr, tol * tol, rr_new));
-        RSATB_CUDA_TRY(cudaMemcpyAsync(hbuf[k & 1], rr_new, sizeof(double) * dw,
-                                       cudaMemcpyDeviceToHost, s.ctx->stream));
+        RSATB_TRY(update(s, w, X, rr, tol * tol, rr_new, hbuf[k & 1]));
         RSATB_CUDA_TRY(cudaEventRecord(ev[k & 1], s.ctx->stream));
         RSATB_TRY(direction(s, w, rr, rr_new));
         std::swap(rr, rr_new);
@@ -441,7 +450,7 @@ int solve_setup(rsatb_context* ctx, const rsatb_bsr_matrix* S, int vdt, int n_ve
     const size_t vb = (s->vbytes + 255) & ~size_t(255);
     const int subs = kDotThreads / n_vectors;
     w->grid = int(std::max<int64_t>(1, std::min<int64_t>((s->n_rows + subs - 1) / subs,
-                                                         int64_t(ctx->sm_count) * 2)));
+                                                         int64_t(ctx->sm_count) * 4)));
     // CTA partials of the fused step kernels' dots (at most sm_count x 8
     // CTAs, two dots of W values) and of the update kernel (grid x R).
     const size_t part_b =
