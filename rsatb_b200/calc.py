@@ -111,6 +111,7 @@ class Chebyshev:
         else:
             self.form = ChebyOpForm.Sandwich if preconditioner is not None else ChebyOpForm.Orthogonal
         self.verbose = verbose
+        self._c_op = self._c_key = None
         self.set_window(emin, emax)
 
     def set_window(self, emin: float, emax: float) -> None:
@@ -140,6 +141,18 @@ class Chebyshev:
         return c
 
     def c_op(self) -> _capi.ChebOp:
+        """The C operator of this object's present matrices, window and solver
+        settings; the last one is reused while none of them is another."""
+        pre = self.M
+        key = (self.form, self.H.handle, None if pre is None else (pre.Z.handle, pre.ZH.handle),
+               None if self.S is None else self.S.handle, self.center, self.half_width,
+               self.cg_tol, self.cg_max_iter)
+        if key == self._c_key:
+            return self._c_op
+        self._c_op, self._c_key = self._make_c_op(), key
+        return self._c_op
+
+    def _make_c_op(self) -> _capi.ChebOp:
         op = _capi.ChebOp()
         op.form = {ChebyOpForm.Sandwich: _capi.FORM_SANDWICH, ChebyOpForm.Solve: _capi.FORM_SOLVE,
                    ChebyOpForm.Orthogonal: _capi.FORM_ORTHOGONAL}[self.form]
@@ -163,8 +176,7 @@ class Chebyshev:
         ctx = self.H.ctx
         ctx.bind_stream()
         op = self.c_op()
-        check(lib().rsatb_cheb_apply_op(ctx.handle, C.byref(op), C.c_void_p(X.data_ptr()),
-                                        C.c_void_p(Y.data_ptr()), X.shape[1],
+        check(lib().rsatb_cheb_apply_op(ctx.handle, op, X.data_ptr(), Y.data_ptr(), X.shape[1],
                                         dtype_code(X.dtype)))
         return Y
 
