@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(256) sddmm_kernel(int n_block_rows, const int3
     }
 }
 
-// The same sampled products on the FP64 tensor cores, blocks of 4 to 8: the
+// The same sampled products on the FP64 tensor cores, blocks of 4, 5 and 8: the
 // sum over (moment, sample) is the contraction index k' = q R + s of
 // mma.sync m8n8k4 tiles.  The tile rows are the block's rows (dropped beyond b),
 // the tile columns run over the columns of all the block row's blocks, so blocks
@@ -200,10 +200,10 @@ template <typename VT>
 int launch_sddmm(rsatb_context* ctx, const rsatb_bsr_matrix* H, int R, int n0, int len,
                  int n_last, double scale, const VT* L, const VT* T, int64_t panel,
                  double* grad) {
-    // Blocks of 4 to 8 fill the 8 x 8 tiles from a quarter up; below that the
-    // warp-per-row kernel does no zero work.
+    // Blocks of 4, 5 and 8 fill the 8 x 8 tiles from a half up; below that the
+    // warp-per-row kernel does no zero work.  Other sizes are refused below.
     const int used = std::min(len, n_last - n0 + 1);
-    if (H->block_size >= 4 && H->block_size <= 8) {
+    if (H->block_size == 4 || H->block_size == 5 || H->block_size == 8) {
         if (used <= 0 || H->nnz_blocks == 0) return RSATB_SUCCESS;
         const int chunks = (std::max(1, H->max_row_blocks) * H->block_size + 8 * kSdTiles - 1) /
                            (8 * kSdTiles);

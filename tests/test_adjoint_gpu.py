@@ -253,3 +253,18 @@ def test_dos_loss_gradient_in_h_and_s_against_finite_differences(torch_cuda):
 
     fd = (L(h) - L(-h)) / (2 * h)
     assert abs(fd - analytic) <= 1e-5 * max(abs(fd), 1e-12), (fd, analytic)
+
+
+@pytest.mark.parametrize("b", [6, 7])
+def test_block_sizes_without_a_gradient_kernel_are_refused(torch_cuda, b):
+    from _util import random_hermitian_bsr
+    from rsatb_b200 import _capi
+    from rsatb_b200.adjoint import kpm_moments_vjp
+    from rsatb_b200.calc import Chebyshev
+    from rsatb_b200.vbcsr import BlockSpMat
+    torch = torch_cuda
+    A = random_hermitian_bsr(9, b, 3, seed=b, complex_values=False, scale=0.1)
+    c = Chebyshev(BlockSpMat(A.row_ptr, A.col_ind, A.values, b), -5.0, 5.0)
+    psi = torch.ones(9 * b, 2, dtype=torch.float64, device="cuda")
+    with pytest.raises(_capi.RsatbError, match="not built"):
+        kpm_moments_vjp(c, psi, 6, np.ones(6))
