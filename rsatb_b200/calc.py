@@ -111,7 +111,7 @@ class Chebyshev:
         else:
             self.form = ChebyOpForm.Sandwich if preconditioner is not None else ChebyOpForm.Orthogonal
         self.verbose = verbose
-        self._c_op = self._c_key = None
+        self._kept_op = (None, None)
         self.set_window(emin, emax)
 
     def set_window(self, emin: float, emax: float) -> None:
@@ -140,19 +140,23 @@ class Chebyshev:
                       cg_tol=self.cg_tol, cg_max_iter=self.cg_max_iter)
         return c
 
-    def c_op(self) -> _capi.ChebOp:
-        """The C operator of this object's present matrices, window and solver
-        settings; the last one is reused while none of them is another."""
+    def _op(self) -> _capi.ChebOp:
+        """c_op for this module's own calls, which do not change it: the last one,
+        while the matrices, the window and the solver settings (all that it
+        holds) are the same."""
         pre = self.M
         key = (self.form, self.H.handle, None if pre is None else (pre.Z.handle, pre.ZH.handle),
                None if self.S is None else self.S.handle, self.center, self.half_width,
                self.cg_tol, self.cg_max_iter)
-        if key == self._c_key:
-            return self._c_op
-        self._c_op, self._c_key = self._make_c_op(), key
-        return self._c_op
+        kept_key, op = self._kept_op  # one attribute: a pair is read and replaced whole
+        if kept_key != key:
+            op = self.c_op()
+            self._kept_op = (key, op)
+        return op
 
-    def _make_c_op(self) -> _capi.ChebOp:
+    def c_op(self) -> _capi.ChebOp:
+        """A C operator of the caller's own, of the present matrices, window and
+        solver settings."""
         op = _capi.ChebOp()
         op.form = {ChebyOpForm.Sandwich: _capi.FORM_SANDWICH, ChebyOpForm.Solve: _capi.FORM_SOLVE,
                    ChebyOpForm.Orthogonal: _capi.FORM_ORTHOGONAL}[self.form]
@@ -175,7 +179,7 @@ class Chebyshev:
             raise NotImplementedError("the Solve form serves NORMAL applications only")
         ctx = self.H.ctx
         ctx.bind_stream()
-        op = self.c_op()
+        op = self._op()
         check(lib().rsatb_cheb_apply_op(ctx.handle, op, X.data_ptr(), Y.data_ptr(), X.shape[1],
                                         dtype_code(X.dtype)))
         return Y
