@@ -64,14 +64,15 @@ void free_matrix(rsatb_bsr_matrix* A) {
 }
 
 // Allocates an empty matrix shell with device arrays of the right size.
-int alloc_matrix(int device, int nbr, int nbc, int b, int64_t nnzb, int dtype, unsigned flags,
-                 rsatb_bsr_matrix** out) {
+int alloc_matrix(int device, int nbr, int nbc, int b, int64_t nnzb, int max_row, int dtype,
+                 unsigned flags, rsatb_bsr_matrix** out) {
     auto* A = new rsatb_bsr_matrix();
     A->device = device;
     A->n_block_rows = nbr;
     A->n_block_cols = nbc;
     A->block_size = b;
     A->nnz_blocks = nnzb;
+    A->max_row_blocks = max_row;
     A->dtype = dtype;
     A->flags = flags & RSATB_BSR_IMAGINARY_UNIT;
     cudaError_t e1 = cudaMalloc(&A->row_ptr, sizeof(int32_t) * (size_t(nbr) + 1));
@@ -143,9 +144,8 @@ int rsatb_bsr_create(rsatb_ctx_t ctx, int n_block_rows, int n_block_cols, int bl
     }
 
     rsatb_bsr_matrix* A = nullptr;
-    RSATB_TRY(alloc_matrix(ctx->device, n_block_rows, n_block_cols, block_size, nnz_blocks, dtype,
-                           flags, &A));
-    A->max_row_blocks = max_row;
+    RSATB_TRY(alloc_matrix(ctx->device, n_block_rows, n_block_cols, block_size, nnz_blocks,
+                           max_row, dtype, flags, &A));
     const size_t vbytes = dtype_size(dtype) * size_t(nnz_blocks) * block_size * block_size;
     cudaError_t err = cudaMemcpy(A->row_ptr, h_ptr.data(), sizeof(int32_t) * h_ptr.size(),
                                  cudaMemcpyHostToDevice);
@@ -245,8 +245,7 @@ int rsatb_bsr_adjoint(rsatb_ctx_t ctx, rsatb_bsr_t A, rsatb_bsr_t* out) {
     for (int j = 0; j < nbc; ++j) max_row = std::max(max_row, tptr[j + 1] - tptr[j]);
 
     rsatb_bsr_matrix* T = nullptr;
-    RSATB_TRY(alloc_matrix(ctx->device, nbc, nbr, b, nnzb, A->dtype, A->flags, &T));
-    T->max_row_blocks = max_row;
+    RSATB_TRY(alloc_matrix(ctx->device, nbc, nbr, b, nnzb, max_row, A->dtype, A->flags, &T));
     int64_t* d_src = nullptr;
     cudaError_t err = cudaMemcpy(T->row_ptr, tptr.data(), sizeof(int32_t) * tptr.size(),
                                  cudaMemcpyHostToDevice);
@@ -323,9 +322,8 @@ int rsatb_bsr_convert(rsatb_ctx_t ctx, rsatb_bsr_t A, rsatb_dtype dtype, rsatb_b
                          (int)dtype);
     const int b = A->block_size;
     rsatb_bsr_matrix* T = nullptr;
-    RSATB_TRY(alloc_matrix(ctx->device, A->n_block_rows, A->n_block_cols, b, A->nnz_blocks, dtype,
-                           A->flags, &T));
-    T->max_row_blocks = A->max_row_blocks;
+    RSATB_TRY(alloc_matrix(ctx->device, A->n_block_rows, A->n_block_cols, b, A->nnz_blocks,
+                           A->max_row_blocks, dtype, A->flags, &T));
     cudaError_t err = cudaMemcpyAsync(T->row_ptr, A->row_ptr,
                                       sizeof(int32_t) * (size_t(A->n_block_rows) + 1),
                                       cudaMemcpyDeviceToDevice, ctx->stream);

@@ -100,7 +100,7 @@ struct rsatb_bsr_matrix {
     void* values = nullptr;       // device
     int dtype = RSATB_F64;
     unsigned flags = 0;           // only RSATB_BSR_IMAGINARY_UNIT is kept
-    int max_row_blocks = 0;
+    int max_row_blocks = 0;       // blocks of the longest row (launches are sized by it)
 };
 
 namespace rsatb_b200 {
@@ -139,9 +139,9 @@ int check_ctx(rsatb_context* ctx);
 int check_bsr(const rsatb_bsr_matrix* A, const char* name);
 
 // A matrix shell with device arrays for nnzb blocks (row_ptr, col_ind and
-// values left unset), and its release.
-int alloc_matrix(int device, int nbr, int nbc, int b, int64_t nnzb, int dtype, unsigned flags,
-                 rsatb_bsr_matrix** out);
+// values left unset), the longest row of max_row blocks; and its release.
+int alloc_matrix(int device, int nbr, int nbc, int b, int64_t nnzb, int max_row, int dtype,
+                 unsigned flags, rsatb_bsr_matrix** out);
 void free_matrix(rsatb_bsr_matrix* A);
 
 }  // namespace rsatb_b200

@@ -367,9 +367,9 @@ int launch_check(rsatb_context* ctx) {
 }
 
 // Host exclusive sum of n device counts into a device row pointer; *total
-// receives the sum.
+// receives the sum, *longest the largest count.
 int offsets_from_counts(rsatb_context* ctx, const int32_t* d_counts, int n, int32_t* d_rp,
-                        int64_t* total) {
+                        int64_t* total, int* longest) {
     std::vector<int32_t> c(static_cast<size_t>(n));
     std::vector<int32_t> rp(static_cast<size_t>(n) + 1);
     if (n)
@@ -377,9 +377,11 @@ int offsets_from_counts(rsatb_context* ctx, const int32_t* d_counts, int n, int3
                                        cudaMemcpyDeviceToHost, ctx->stream));
     RSATB_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     int64_t s = 0;
+    *longest = 0;
     for (int i = 0; i < n; ++i) {
         rp[i] = int32_t(s);
         s += c[i];
+        *longest = std::max(*longest, int(c[i]));
         if (s > INT32_MAX)
             return set_error(RSATB_OUT_OF_MEMORY, "sparse product exceeds 2^31 blocks");
     }
@@ -429,8 +431,10 @@ int spgemm(rsatb_context* ctx, const rsatb_bsr_matrix* A, const rsatb_bsr_matrix
     DevBuf rp_tmp;
     RSATB_TRY(dev_alloc(rp_tmp, sizeof(int32_t) * (size_t(n) + 1)));
     int64_t nnz = 0;
-    RSATB_TRY(offsets_from_counts(ctx, counts.as<int32_t>(), n, rp_tmp.as<int32_t>(), &nnz));
-    RSATB_TRY(alloc_matrix(ctx->device, n, nbc, b, nnz, RSATB_F64, 0, &raw));
+    int longest = 0;
+    RSATB_TRY(offsets_from_counts(ctx, counts.as<int32_t>(), n, rp_tmp.as<int32_t>(), &nnz,
+                                  &longest));
+    RSATB_TRY(alloc_matrix(ctx->device, n, nbc, b, nnz, longest, RSATB_F64, 0, &raw));
     Mat C(raw);
     RSATB_CUDA_TRY(cudaMemcpyAsync(C->row_ptr, rp_tmp.p, sizeof(int32_t) * (size_t(n) + 1),
                                    cudaMemcpyDeviceToDevice, ctx->stream));
@@ -475,9 +479,10 @@ int spgemm(rsatb_context* ctx, const rsatb_bsr_matrix* A, const rsatb_bsr_matrix
         n, C->row_ptr, keep.as<uint8_t>(), newpos.as<int32_t>(), counts.as<int32_t>());
     RSATB_TRY(launch_check(ctx));
     int64_t kept = 0;
-    RSATB_TRY(offsets_from_counts(ctx, counts.as<int32_t>(), n, rp_tmp.as<int32_t>(), &kept));
+    RSATB_TRY(offsets_from_counts(ctx, counts.as<int32_t>(), n, rp_tmp.as<int32_t>(), &kept,
+                                  &longest));
     rsatb_bsr_matrix* raw2 = nullptr;
-    RSATB_TRY(alloc_matrix(ctx->device, n, nbc, b, kept, RSATB_F64, 0, &raw2));
+    RSATB_TRY(alloc_matrix(ctx->device, n, nbc, b, kept, longest, RSATB_F64, 0, &raw2));
     Mat K(raw2);
     RSATB_CUDA_TRY(cudaMemcpyAsync(K->row_ptr, rp_tmp.p, sizeof(int32_t) * (size_t(n) + 1),
                                    cudaMemcpyDeviceToDevice, ctx->stream));
@@ -532,7 +537,7 @@ int products(rsatb_context* ctx, const rsatb_bsr_matrix* A, const rsatb_bsr_matr
 int copy_matrix(rsatb_context* ctx, const rsatb_bsr_matrix* A, Mat* out) {
     rsatb_bsr_matrix* raw = nullptr;
     RSATB_TRY(alloc_matrix(ctx->device, A->n_block_rows, A->n_block_cols, A->block_size,
-                           A->nnz_blocks, RSATB_F64, 0, &raw));
+                           A->nnz_blocks, A->max_row_blocks, RSATB_F64, 0, &raw));
     Mat C(raw);
     const size_t bb = size_t(A->block_size) * A->block_size;
     RSATB_CUDA_TRY(cudaMemcpyAsync(C->row_ptr, A->row_ptr,

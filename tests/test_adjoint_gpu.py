@@ -268,3 +268,33 @@ def test_block_sizes_without_a_gradient_kernel_are_refused(torch_cuda, b):
     psi = torch.ones(9 * b, 2, dtype=torch.float64, device="cuda")
     with pytest.raises(_capi.RsatbError, match="not built"):
         kpm_moments_vjp(c, psi, 6, np.ones(6))
+
+
+@pytest.mark.parametrize("stride", [0, 5])
+def test_sandwich_vjp_with_a_refined_preconditioner(torch_cuda, stride):
+    """Z from the sparse refinement, whose pattern the library grows: rows of more
+    8 x 8 blocks than one warp's columns of a gradient row (48) take every block."""
+    torch = torch_cuda
+    from rsatb_b200 import lattice
+    from rsatb_b200.adjoint import kpm_moments_vjp_sandwich
+    from rsatb_b200.calc import Chebyshev, ISQRTMPreconditioner
+    from rsatb_b200.isqrt import InverseSqrtOptions, inverse_sqrt
+    from rsatb_b200.vbcsr import BlockSpMat
+    H, S = lattice.diamond_lcao(L=2, seed=3)
+    Zd, _ = inverse_sqrt(S, InverseSqrtOptions(tol=1e-11, sptol=1e-9, maxit=12))
+    Z = Zd.to_arrays()
+    assert np.diff(Z.row_ptr).max() * 8 > 48
+    Hm, Zm = H.to_dense(), Z.to_dense()
+    w = np.linalg.eigvalsh(Zm.T @ Hm @ Zm)
+    emin, emax = w[0] - 0.5, w[-1] + 0.5
+    c, hw = (emax + emin) / 2, (emax - emin) / 2
+    cheby = Chebyshev(BlockSpMat(H.row_ptr, H.col_ind, H.values, 8), emin, emax,
+                      preconditioner=ISQRTMPreconditioner(Zd))
+    M = 24
+    psi = np.random.default_rng(9).choice([-1.0, 1.0], (H.n_rows, 6)) / np.sqrt(H.n_rows)
+    dmu = np.random.default_rng(10).standard_normal(M)
+    gh, gz, _, _ = kpm_moments_vjp_sandwich(cheby, torch.as_tensor(psi).cuda(), M, dmu,
+                                            checkpoint_stride=stride)
+    Gs = oracle.kpm_moments_vjp_dense(Zm.T @ Hm @ Zm, psi, c, hw, M, dmu)
+    assert rel_err(gh.cpu().numpy(), _on_pattern(H, Zm @ Gs @ Zm.T)) < 1e-10
+    assert rel_err(gz.cpu().numpy(), _on_pattern(Z, Hm @ Zm @ (Gs + Gs.T))) < 1e-10
