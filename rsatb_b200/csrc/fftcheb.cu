@@ -27,6 +27,7 @@
 //   hand-written kernel after a coalesced gather: transform and contraction
 //   without the FP64 extension buffer's round trips (greenwood_fused_kernel).
 #include "cheb_kernels.cuh"
+#include "fftcheb_partition.cuh"
 
 #include <cufft.h>
 
@@ -1153,9 +1154,6 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
                  int formulation, double prefactor, int sections, size_t workspace, int kernel,
                  double* sigma_out, double* energy_out, rsatb_fftcheb_stats* stats) {
     const bool bastin = formulation == 1;
-    // Transform points per side and sequence: the M-point DCT-III, or Bastin's
-    // zero-padded 2M-point phi1 and phi2 (phi3 comes out of phi1).
-    const int n_pts = bastin ? 4 * M : M;
     rsatb_context* ctx = c.ctx;
     cudaStream_t st = ctx->stream;
     const int b = c.op->H->block_size;
@@ -1164,8 +1162,6 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
     const int W1 = 2 * R, W3 = 6 * R;  // real values per row: left, right panel
     const size_t cplx = 2 * sizeof(T);
 
-    // Store per block row: both chains, all moments, 3 axes x R samples.
-    const size_t store_per_brow = 2 * size_t(M) * b * 3 * R * cplx;
     size_t fixed = size_t(N) * cplx * (3 * R /*rinit*/ + 3 * 3 * R /*r*/ + 3 * R /*l*/ +
                                       3 * R /*J psi*/ + (c.sandwich ? 2 * 3 * R : 0));
     if (workspace == 0) {
@@ -1206,37 +1202,24 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
         else
             fixed = fixed_m;
     }
-    if (workspace <= fixed + store_per_brow)
-        return set_error(RSATB_OUT_OF_MEMORY,
-                         "workspace of %zu bytes holds no section (needs %zu + %zu per block row)",
-                         workspace, fixed, store_per_brow);
-    // FFT chunk: rows whose 2 x (2M x 3 rows R) double2 extensions fit a
-    // quarter of what remains after the fixed buffers.  The fused row stage
-    // (Greenwood, fused_radix) needs only its gathered chunk of up to 8,192
-    // sequence pairs, and the store takes the rest (larger sections: fewer
-    // passes of the recurrence).
-    const size_t avail = workspace - fixed;
     const int radix = bastin ? 0 : fused_radix(M);
     const bool fused = radix && fused_enabled();
-    const size_t fused_chunk_bytes = 2 * size_t(8192) * size_t(M) * cplx;
-    const size_t fft_budget =
-        fused ? std::max(2 * size_t(M) * cplx, std::min(avail / 4, fused_chunk_bytes))
-              : std::min(avail / 4, size_t(2) << 30);
-    const size_t fft_per_row =
-        2 * size_t(n_pts) * 3 * R * sizeof(double2) * 2;  // + cuFFT work
-    int64_t chunk_rows = int64_t(fft_budget / fft_per_row);
-    if (chunk_rows < 1) chunk_rows = 1;
-    int64_t sec_brows = int64_t((avail - fft_budget) / store_per_brow);
-    if (sec_brows < 1)
-        return set_error(RSATB_OUT_OF_MEMORY, "workspace too small for one block row of stores");
-    if (sections > 0) {
-        const int64_t want = (nb + sections - 1) / sections;
-        if (want < sec_brows) sec_brows = want;
+    const FftchebSizes sizes{workspace, fixed,  nb,    b,        R, M, cplx,
+                             bastin,    fused, sections};
+    FftchebPartition part{};
+    switch (fftcheb_partition(sizes, &part)) {
+        case FftchebFit::kNoSection:
+            return set_error(
+                RSATB_OUT_OF_MEMORY,
+                "workspace of %zu bytes holds no section (needs %zu + %zu per block row)",
+                workspace, fixed, fftcheb_store_per_brow(sizes));
+        case FftchebFit::kNoRow:
+            return set_error(RSATB_OUT_OF_MEMORY,
+                             "workspace too small for one block row of stores");
+        case FftchebFit::kFits: break;
     }
-    if (sec_brows > nb) sec_brows = nb;
-    const int n_sections = int((nb + sec_brows - 1) / sec_brows);
-    sec_brows = (nb + n_sections - 1) / n_sections;  // balanced: the store is no larger than needed
-    if (chunk_rows > sec_brows * b) chunk_rows = sec_brows * b;
+    const int64_t sec_brows = part.sec_brows, chunk_rows = part.chunk_rows;
+    const int n_sections = part.n_sections;
 
     // Buffers.
     Arena mem;
@@ -1245,7 +1228,7 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
     const int64_t sec_rows_max = sec_brows * b;
     const int64_t slot = 3 * sec_rows_max * R;  // complex entries per moment slot
     const int64_t nq_max = 3 * chunk_rows * R;
-    const size_t e_bytes = fused ? fft_budget : 2 * size_t(n_pts) * nq_max * sizeof(double2);
+    const size_t e_bytes = part.e_bytes;
     const size_t oPan = one_launch ? mem.reserve(2 * panel * sizeof(T)) : 0;
     const size_t oInit = one_launch ? mem.reserve(panel * sizeof(T)) : 0;
     const size_t oJ = one_launch ? 0 : mem.reserve(3 * v1);
