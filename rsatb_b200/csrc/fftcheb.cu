@@ -1162,7 +1162,7 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
     const int W1 = 2 * R, W3 = 6 * R;  // real values per row: left, right panel
     const size_t cplx = 2 * sizeof(T);
 
-    size_t fixed = size_t(N) * cplx * (3 * R /*rinit*/ + 3 * 3 * R /*r*/ + 3 * R /*l*/ +
+    const size_t fixed = size_t(N) * cplx * (3 * R /*rinit*/ + 3 * 3 * R /*r*/ + 3 * R /*l*/ +
                                       3 * R /*J psi*/ + (c.sandwich ? 2 * 3 * R : 0));
     if (workspace == 0) {
         size_t free_b = 0, total_b = 0;
@@ -1171,14 +1171,23 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
     }
     // One launch per moment (moment_kernel) where the four matrices allow it
     // and its buffers (two panels, the start, the packed values) are no larger
-    // than the separate launches' or small in the workspace; RSATB_FFTCHEB_MOMENT=0
-    // keeps the separate launches.
+    // than the separate launches' or small in the workspace, and a section still
+    // fits beside them; RSATB_FFTCHEB_MOMENT=0 keeps the separate launches.
+    const int radix = bastin ? 0 : fused_radix(M);
+    const bool fused = radix && fused_enabled();
+    FftchebSizes sizes{workspace, fixed, nb, b, R, M, cplx, bastin, fused, sections};
+    FftchebPartition part{};
     T* wgt = nullptr;  // in the context's scratch
     const int64_t nnz = c.op->H->nnz_blocks;
     const size_t fixed_m =
         size_t(N) * cplx * 3 * 4 * R + 4 * size_t(nnz) * sizeof(T) + sizeof(int) + 256;
     bool one_launch = moment_enabled() && moment_matrices_ok(c, V, R) &&
                       fixed_m <= std::max(fixed, workspace / 8);
+    if (one_launch) {
+        sizes.fixed = fixed_m;
+        one_launch = fftcheb_partition(sizes, &part) == FftchebFit::kFits;
+        sizes.fixed = fixed;
+    }
     if (one_launch) {
         void* sc = nullptr;
         RSATB_TRY(ctx_scratch(ctx, 4 * size_t(nnz) * sizeof(T) + 256, &sc));
@@ -1200,19 +1209,14 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
         if (differs)
             one_launch = false;
         else
-            fixed = fixed_m;
+            sizes.fixed = fixed_m;
     }
-    const int radix = bastin ? 0 : fused_radix(M);
-    const bool fused = radix && fused_enabled();
-    const FftchebSizes sizes{workspace, fixed,  nb,    b,        R, M, cplx,
-                             bastin,    fused, sections};
-    FftchebPartition part{};
     switch (fftcheb_partition(sizes, &part)) {
         case FftchebFit::kNoSection:
             return set_error(
                 RSATB_OUT_OF_MEMORY,
                 "workspace of %zu bytes holds no section (needs %zu + %zu per block row)",
-                workspace, fixed, fftcheb_store_per_brow(sizes));
+                workspace, sizes.fixed, fftcheb_store_per_brow(sizes));
         case FftchebFit::kNoRow:
             return set_error(RSATB_OUT_OF_MEMORY,
                              "workspace too small for one block row of stores");

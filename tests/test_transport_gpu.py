@@ -304,12 +304,12 @@ def test_fused_row_stage_at_2048_moments(torch_cuda, precision, monkeypatch):
         assert rel_err(fused, sig_o) < 1e-10
 
 
-def _scalar_chain(n, long_row, seed):
+def _scalar_chain(n, long_row, seed, full=False):
     """A real symmetric scalar-row H on a ring with one row of long_row
-    nonzeros, and real antisymmetric W_a on the same pattern."""
+    nonzeros (full: every row), and real antisymmetric W_a on the same pattern."""
     from rsatb_b200 import lattice
     rng = np.random.default_rng(seed)
-    A = np.zeros((n, n), dtype=bool)
+    A = np.full((n, n), full)
     i = np.arange(n)
     A[i, (i + 1) % n] = A[i, i] = True
     A[3, rng.permutation(n)[:long_row]] = True
@@ -371,3 +371,22 @@ def test_velocity_of_another_pattern_keeps_the_separate_launches(torch_cuda):
     psi = _phases(n, 3, seed=6)
     sig = _gpu(torch_cuda, H, V, psi, 24, -8.0, 8.0)[0]
     assert rel_err(sig, _oracle(H, V, psi, 24, -8.0, 8.0)[0]) < 1e-10
+
+
+def test_a_workspace_that_holds_the_separate_launches_is_accepted(torch_cuda):
+    """16 dense rows, one sample: the one-launch buffers (values of four matrices)
+    are larger than the separate launches' panels.  A bound that holds one row's
+    store beside the latter only takes the separate launches."""
+    n, M = 16, 650
+    H, V = _scalar_chain(n, n, seed=5, full=True)
+    assert H.nnz_blocks == n * n
+    psi = _phases(n, 1, seed=4)
+    kw = dict(torch=torch_cuda, H=H, V=V, psi=psi, M=M, emin=-8.0, emax=8.0)
+    sep = n * 16 * 18                     # panels of the separate launches
+    one = n * 16 * 12 + 4 * n * n * 8     # panels and packed values of the one launch
+    store = 2 * M * 3 * 16                # one row's moments
+    ws = 93_000
+    assert one < ws / 8 and 0.75 * (ws - one) < store < 0.75 * (ws - sep)
+    sig, _, st = _gpu(**kw, max_workspace_mb=ws / (1 << 20))
+    assert st["sections"] == n
+    assert rel_err(sig, _gpu(**kw)[0]) < 1e-12
