@@ -1175,7 +1175,9 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
     // fits beside them; RSATB_FFTCHEB_MOMENT=0 keeps the separate launches.
     const int radix = bastin ? 0 : fused_radix(M);
     const bool fused = radix && fused_enabled();
-    FftchebSizes sizes{workspace, fixed, nb, b, R, M, cplx, bastin, fused, sections};
+    const size_t part_bytes = fused ? fused_pairs(radix) * size_t(M) * sizeof(double2) : 0;
+    FftchebSizes sizes{workspace, fixed,      nb, b, R, M, cplx, bastin,
+                       part_bytes, ctx->sm_count * 2, sections};
     FftchebPartition part{};
     T* wgt = nullptr;  // in the context's scratch
     const int64_t nnz = c.op->H->nnz_blocks;
@@ -1246,14 +1248,14 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
     const size_t oK = mem.reserve(size_t(M) * 12 * sizeof(double));
     const size_t oWts = mem.reserve(size_t(M) * sizeof(double));
     const size_t oPw = bastin ? mem.reserve(2 * size_t(M) * sizeof(double2)) : 0;
-    // Fused row stage: two CTAs per SM, partial sums per CTA, pair of sequences
+    // Fused row stage: up to two CTAs per SM, partial sums per CTA, pair of sequences
     // and energy; chunks of fused_qc sequences gathered into the extension
     // buffer (sequence-major, both sides).  FP32 vectors take the FP32
     // transform at M = 2048 (FP64 products and sums) unless
     // RSATB_FFTCHEB_FP64=1; every other case the FP64 one.
     const bool fused32 = fused && M == 2048 && std::is_same<T, float>::value &&
                          !fused_fp64_forced();
-    const int fused_grid = ctx->sm_count * 2;
+    const int fused_grid = part.ctas;
     const int n_part = fused ? fused_grid * fused_pairs(radix) : 0;
     const size_t oPart = fused ? mem.reserve(size_t(n_part) * M * sizeof(double2)) : 0;
     const size_t oTab = fused ? mem.reserve(size_t(M / 4 + M) * sizeof(double2)) : 0;

@@ -22,12 +22,12 @@ def partition(tmp_path_factory):
                    check=True, capture_output=True, text=True)
 
     def ask(cases):
-        keys = ("workspace", "fixed", "brows", "b", "R", "M", "cplx", "bastin", "fused", "sections")
+        keys = ("workspace", "fixed", "brows", "b", "R", "M", "cplx", "bastin", "part", "sections")
         text = "\n".join(" ".join(str(int(c[k])) for k in keys) for c in cases)
         out = subprocess.run([str(exe)], input=text, check=True, capture_output=True, text=True)
         rows = [list(map(int, line.split())) for line in out.stdout.splitlines()]
         assert len(rows) == len(cases)
-        names = ("fit", "sec_brows", "sections", "chunk_rows", "e_bytes")
+        names = ("fit", "sec_brows", "sections", "chunk_rows", "e_bytes", "ctas")
         return [dict(zip(names, r)) for r in rows]
 
     return ask
@@ -43,15 +43,15 @@ def _per_row(c):
 
 
 def _held(c, p):
-    work = 1 if c["fused"] else 2
-    return c["fixed"] + p["sec_brows"] * _store(c) + work * p["e_bytes"]
+    row_stage = p["e_bytes"] + p["ctas"] * c["part"] if c["part"] else 2 * p["e_bytes"]
+    return c["fixed"] + p["sec_brows"] * _store(c) + row_stage
 
 
 def test_a_row_of_more_than_the_cap_stays_within_the_bound(partition):
     """Bastin, 256 samples, 12,000 moments: one row's transforms are 2.2 GB, more
     than the stage's usual share, and the workspace's quarter holds them."""
     c = dict(workspace=12 * GB, fixed=GB // 4, brows=1000, b=1, R=256, M=12000, cplx=16,
-             bastin=1, fused=0, sections=0)
+             bastin=1, part=0, sections=0)
     assert 2 * GB < _per_row(c) < (c["workspace"] - c["fixed"]) // 4
     p, = partition([c])
     assert p["fit"] == 0 and p["chunk_rows"] == 1
@@ -75,7 +75,7 @@ def test_bounds_over_random_shapes(partition):
         if fused:
             M = int(rng.choice([256, 512, 1024, 2048]))
         c = dict(b=int(rng.choice([1, 4, 5, 8, 13])), R=int(np.exp(rng.uniform(0, np.log(256)))),
-                 M=M, cplx=int(rng.choice([8, 16])), fused=fused,
+                 M=M, cplx=int(rng.choice([8, 16])), part=fused * 8 * 256 * 16,
                  bastin=0 if fused else int(rng.random() < 0.5),
                  brows=int(np.exp(rng.uniform(0, np.log(200000)))),
                  sections=int(rng.choice([0, 0, 1, 3])))
@@ -91,6 +91,13 @@ def test_bounds_over_random_shapes(partition):
         fits += 1
         assert 1 <= p["sec_brows"] <= c["brows"] and p["chunk_rows"] >= 1
         assert p["sections"] * p["sec_brows"] >= c["brows"] > (p["sections"] - 1) * p["sec_brows"]
-        if c["fused"] or _per_row(c) <= (c["workspace"] - c["fixed"]) // 4:
+        if c["part"]:
+            # beyond the bound by a pair of sequences and one CTA's sums at most,
+            # where one block row's stores take all but less than these
+            spare = c["workspace"] - c["fixed"] - _store(c)
+            least = 2 * c["M"] * c["cplx"] + c["part"]
+            assert p["ctas"] >= 1 and p["e_bytes"] >= 2 * c["M"] * c["cplx"]
+            assert _held(c, p) <= c["workspace"] + (least if spare < 2 * least else 0), (c, p)
+        elif _per_row(c) <= (c["workspace"] - c["fixed"]) // 4:
             assert _held(c, p) <= c["workspace"], (c, p)
     assert fits > 2000
