@@ -119,6 +119,11 @@ RSATB_API void* rsatb_ctx_stream(rsatb_ctx_t ctx);
  * entry point that synchronises (moments, transport, CG, the adjoint)
  * reports such a give-up the same way, its own or an earlier call's. */
 RSATB_API int rsatb_ctx_synchronize(rsatb_ctx_t ctx);
+/* Gives back the device memory and FFT plans that rsatb_dc_spectrum_fftcheb keeps
+ * for the context's next call (at most 1/16 of the device's memory).  It need not
+ * be called to make room inside the process: a failing cudaMalloc there takes that
+ * memory back by itself.  Waits for the context's stream. */
+RSATB_API int rsatb_ctx_release_workspace(rsatb_ctx_t ctx);
 /* Number of kernels the context has launched so far (all entry points). */
 RSATB_API int64_t rsatb_ctx_launch_count(rsatb_ctx_t ctx);
 
@@ -414,15 +419,19 @@ typedef struct {
  * K(E_k) = sum conj(L3) R3 / max(1e-14, 1 - eps_k^2), averaged over the
  * samples.  Vx, Vy, Vz: velocity matrices (RSATB_BSR_IMAGINARY_UNIT for the
  * i*W of a real k-point, or complex), H's shape and precision.  psi: device
- * N x n_vectors complex (C128, or C64 for FP32 vectors; the transform and
- * the contraction are FP64 either way).  formulation 0 Greenwood, 1
+ * N x n_vectors complex (C128, or C64 for FP32 vectors; the contraction is
+ * FP64 either way, and so is the transform, but for C64 Greenwood at 2048
+ * moments, which transforms in FP32).  formulation 0 Greenwood, 1
  * Bastin: beside phi3 the zero-padded 2M-point inverse FFTs phi1, phi2 of
  * the moments times the complex phase weights (:443-461), all six (a, b)
  * components of eps (conj(L3_a) R1_b + conj(L1_a) R3_b) + i sqrt(1 - eps^2)
  * (conj(L2_a) R3_b - conj(L3_a) R2_b) (:496-519), then the cumulative
  * trapezoid of Re(i zeta) over the ascending grid: sigma(mu, T = 0)
  * (:635-659).  partition_sections > 0 asks for at least that many row sections,
- * max_workspace_bytes bounds the device memory (0: 80 % of what is free).
+ * max_workspace_bytes bounds the device memory of panels, stores and transforms
+ * (0: 80 % of what is free; tables of about 150 bytes per moment come beside it).
+ * Up to 1/16 of the device's memory stays with the context for its next call
+ * (rsatb_ctx_release_workspace).
  * sigma_out (host) receives n_moments x 6 (xx xy xz yy yz zz; Greenwood
  * fills xx, yy, zz) scaled by prefactor, energy_out (host) the ascending
  * energies c + hw cos(pi (M - 1 - k + 1/2) / M).  stats may be NULL.

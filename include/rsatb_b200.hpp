@@ -85,6 +85,7 @@ public:
     Context& operator=(const Context&) = delete;
     rsatb_ctx_t handle() const { return h_; }
     void synchronize() const { check(rsatb_ctx_synchronize(h_)); }
+    void release_workspace() const { check(rsatb_ctx_release_workspace(h_)); }
 
 private:
     rsatb_ctx_t h_ = nullptr;

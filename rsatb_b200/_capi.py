@@ -110,6 +110,7 @@ SIGNATURES = {
     "rsatb_ctx_set_stream": (_i, [_vp, _vp]),
     "rsatb_ctx_stream": (_vp, [_vp]),
     "rsatb_ctx_synchronize": (_i, [_vp]),
+    "rsatb_ctx_release_workspace": (_i, [_vp]),
     "rsatb_ctx_launch_count": (_i64, [_vp]),
     "rsatb_device_alloc": (_i, [_vp, _sz, C.POINTER(_vp)]),
     "rsatb_device_free": (_i, [_vp, _vp]),

@@ -72,11 +72,12 @@ struct rsatb_context {
     std::string kpm_graph_key;
     std::string kpm_seen_key;
     int64_t kpm_graph_launches = 0;
-    // The transport's workspace, kept between calls up to kKeepWorkShare of the
-    // device's memory (larger ones are the call's own), and the last two cuFFT
-    // plans it made (their work areas lie in the workspace).
-    void* work = nullptr;
-    size_t work_bytes = 0;
+    // The pool of the transport's workspace (made at its first use), which keeps
+    // up to work_keep bytes between calls, the last call's workspace, and the last
+    // two cuFFT plans it made (their work areas lie in the workspace).
+    cudaMemPool_t work_pool = nullptr;
+    size_t work_keep = 0;
+    size_t work_last = 0;
     struct FftPlan {
         int handle = 0;
         int n = 0;
@@ -128,6 +129,8 @@ int ctx_counters(rsatb_context* ctx, int n, unsigned** out);
 // The context's device fault word (the last of its 64 counters): kernels
 // whose bounded waits give up set it non-zero.
 int ctx_fault_word(rsatb_context* ctx, unsigned** out);
+// Gives the kept transport workspace and plans back (after the stream's work).
+int ctx_release_work(rsatb_context* ctx);
 // Pinned host memory of at least `bytes` (grow-only, released with the
 // context).
 int ctx_pinned(rsatb_context* ctx, size_t bytes, void** out);

@@ -92,6 +92,17 @@ int ctx_pinned(rsatb_context* ctx, size_t bytes, void** out) {
     return RSATB_SUCCESS;
 }
 
+int ctx_release_work(rsatb_context* ctx) {
+    RSATB_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    if (ctx->work_pool) RSATB_CUDA_TRY(cudaMemPoolTrimTo(ctx->work_pool, 0));
+    ctx->work_last = 0;
+    for (auto& f : ctx->fft) {
+        if (f.batch) cufftDestroy(f.handle);
+        f.batch = 0;
+    }
+    return RSATB_SUCCESS;
+}
+
 int ctx_fault_word(rsatb_context* ctx, unsigned** out) {
     unsigned* c = nullptr;
     RSATB_TRY(ctx_counters(ctx, 1, &c));
@@ -156,9 +167,8 @@ int rsatb_ctx_destroy(rsatb_ctx_t ctx) {
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     if (ctx->scratch) cudaFree(ctx->scratch);
-    if (ctx->work) cudaFree(ctx->work);
-    for (auto& f : ctx->fft)
-        if (f.batch) cufftDestroy(f.handle);
+    ctx_release_work(ctx);
+    if (ctx->work_pool) cudaMemPoolDestroy(ctx->work_pool);
     if (ctx->counters) cudaFree(ctx->counters);
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
     if (ctx->kpm_graph) cudaGraphExecDestroy(ctx->kpm_graph);
@@ -185,6 +195,12 @@ int rsatb_ctx_synchronize(rsatb_ctx_t ctx) {
     // Bounded waits that gave up in asynchronous calls queued on this context
     // (mult_dense, apply_op, apply_dual, propagate) are reported here.
     return ctx_check_fault(ctx);
+}
+
+int rsatb_ctx_release_workspace(rsatb_ctx_t ctx) {
+    clear_error();
+    RSATB_TRY(check_ctx(ctx));
+    return ctx_release_work(ctx);
 }
 
 int64_t rsatb_ctx_launch_count(rsatb_ctx_t ctx) { return ctx ? ctx->launches : 0; }

@@ -319,21 +319,29 @@ __global__ void moment_init_kernel(int64_t n_rows, int R, const int32_t* row_ptr
     }
 }
 
-// {h, w_x, w_y, w_z} per nonzero; *differs becomes non-zero when a velocity's
-// pattern is not H's (the caller then keeps the separate launches).
+// {h, w_x, w_y, w_z} per nonzero.
 template <typename T>
-__global__ void pack_weights_kernel(int64_t n_rows, int64_t nnz, const int32_t* rp,
-                                    const int32_t* ci, const T* h, const int32_t* rpx,
-                                    const int32_t* cix, const T* wx, const int32_t* rpy,
-                                    const int32_t* ciy, const T* wy, const int32_t* rpz,
-                                    const int32_t* ciz, const T* wz, T* wgt, int* differs) {
+__global__ void pack_weights_kernel(int64_t nnz, const T* h, const T* wx, const T* wy,
+                                    const T* wz, T* wgt) {
+    for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < nnz;
+         e += int64_t(gridDim.x) * blockDim.x) {
+        const T v[4] = {h[e], wx[e], wy[e], wz[e]};
+        store_vals<T, 4>(wgt + 4 * e, v);
+    }
+}
+
+// *differs becomes non-zero when a velocity's pattern is not H's (the caller then
+// keeps the separate launches).
+__global__ void compare_patterns_kernel(int64_t n_rows, int64_t nnz, const int32_t* rp,
+                                        const int32_t* ci, const int32_t* rpx,
+                                        const int32_t* cix, const int32_t* rpy,
+                                        const int32_t* ciy, const int32_t* rpz,
+                                        const int32_t* ciz, int* differs) {
     bool bad = false;
     for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < nnz;
          e += int64_t(gridDim.x) * blockDim.x) {
         const int32_t j = ci[e];
         bad |= cix[e] != j || ciy[e] != j || ciz[e] != j;
-        const T v[4] = {h[e], wx[e], wy[e], wz[e]};
-        store_vals<T, 4>(wgt + 4 * e, v);
     }
     for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e <= n_rows;
          e += int64_t(gridDim.x) * blockDim.x) {
@@ -940,40 +948,85 @@ struct DevBuf {
     }
 };
 
-// Device memory of one call: every buffer is a piece of one block, the
-// context's kept one when the call needs at most 1/16 of the device's memory,
-// else one allocation released at the end.  (Ten cudaMalloc / cudaFree pairs
-// per call cost 20 ms at 11 GB, 4 ms at 0.5 GB.)
+// The context's workspace pool, made at its first use: it keeps what calls give
+// back, up to a sixteenth of the device's memory, for the next one.  Memory it
+// keeps stays the process's: the driver takes it back for a cudaMalloc or
+// cuMemCreate that would fail otherwise, whoever calls it.
 constexpr size_t kKeepWorkShare = 16;
 
+int work_pool(rsatb_context* ctx) {
+    if (ctx->work_pool) return RSATB_SUCCESS;
+    size_t free_b = 0, total_b = 0;
+    RSATB_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = ctx->device;
+    cudaMemPool_t pool = nullptr;
+    RSATB_CUDA_TRY(cudaMemPoolCreate(&pool, &props));
+    uint64_t keep = total_b / kKeepWorkShare;
+    const cudaError_t e =
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) cudaMemPoolDestroy(pool);
+    RSATB_CUDA_TRY(e);
+    ctx->work_pool = pool;
+    ctx->work_keep = keep;
+    return RSATB_SUCCESS;
+}
+
+// Bytes the pool holds that no call uses.
+int kept_work(rsatb_context* ctx, size_t* bytes) {
+    uint64_t held = 0, used = 0;
+    *bytes = 0;
+    if (!ctx->work_pool) return RSATB_SUCCESS;
+    RSATB_CUDA_TRY(
+        cudaMemPoolGetAttribute(ctx->work_pool, cudaMemPoolAttrReservedMemCurrent, &held));
+    RSATB_CUDA_TRY(cudaMemPoolGetAttribute(ctx->work_pool, cudaMemPoolAttrUsedMemCurrent, &used));
+    *bytes = size_t(held - used);
+    return RSATB_SUCCESS;
+}
+
+// Device memory of one call: every buffer is a piece of one block, an allocation
+// released at the end, or the pool's for a context that calls again: from the
+// second call in a row of one size on, up to what the pool keeps.  (The block from
+// cudaMalloc and its cudaFree take 10 ms at 11 GB, 0.8 ms at 0.3 GB; out of the
+// pool microseconds, but 65 and 5 ms where the pool maps it anew, so a single
+// call, or calls of ever other sizes, do not go there.)
 class Arena {
   public:
+    ~Arena() {
+        if (!base_) return;
+        if (pooled_) {
+            cudaFreeAsync(base_, stream_);
+            cudaStreamSynchronize(stream_);  // seen as free from here on
+        } else {
+            cudaFree(base_);
+        }
+    }
     size_t reserve(size_t bytes) {
         const size_t at = total_;
         total_ += (std::max<size_t>(bytes, 16) + 255) & ~size_t(255);
         return at;
     }
     int commit(rsatb_context* ctx) {
-        size_t free_b = 0, total_b = 0;
-        if (ctx->work_bytes < total_) {
-            RSATB_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-            if (total_ > total_b / kKeepWorkShare) {
-                // The kept block may be what is missing.
-                cudaError_t e = cudaMalloc(&own_.p, total_);
-                if (e == cudaErrorMemoryAllocation && ctx->work) {
-                    cudaGetLastError();
-                    RSATB_TRY(drop(ctx));
-                    e = cudaMalloc(&own_.p, total_);
-                }
-                RSATB_CUDA_TRY(e);
-                base_ = own_.as<char>();
-                return RSATB_SUCCESS;
-            }
-            RSATB_TRY(drop(ctx));
-            RSATB_CUDA_TRY(cudaMalloc(&ctx->work, total_));
-            ctx->work_bytes = total_;
+        RSATB_TRY(work_pool(ctx));
+        size_t kept = 0;
+        RSATB_TRY(kept_work(ctx, &kept));
+        const bool pooled = total_ <= ctx->work_keep && (kept || total_ == ctx->work_last);
+        ctx->work_last = total_;
+        // A kept block too small for this call is not held beside the new one.
+        if (kept && (!pooled || kept < total_)) {
+            RSATB_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+            RSATB_CUDA_TRY(cudaMemPoolTrimTo(ctx->work_pool, 0));
         }
-        base_ = static_cast<char*>(ctx->work);
+        void* p = nullptr;
+        if (pooled)
+            RSATB_CUDA_TRY(cudaMallocFromPoolAsync(&p, total_, ctx->work_pool, ctx->stream));
+        else
+            RSATB_CUDA_TRY(cudaMalloc(&p, total_));
+        pooled_ = pooled;
+        stream_ = ctx->stream;
+        base_ = static_cast<char*>(p);
         return RSATB_SUCCESS;
     }
     template <typename T>
@@ -982,18 +1035,10 @@ class Arena {
     }
 
   private:
-    static int drop(rsatb_context* ctx) {
-        if (!ctx->work) return RSATB_SUCCESS;
-        RSATB_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-        void* p = ctx->work;
-        ctx->work = nullptr;
-        ctx->work_bytes = 0;
-        RSATB_CUDA_TRY(cudaFree(p));
-        return RSATB_SUCCESS;
-    }
     size_t total_ = 0;
     char* base_ = nullptr;
-    DevBuf own_;
+    bool pooled_ = false;
+    cudaStream_t stream_ = nullptr;
 };
 
 // The context's inverse Z2Z plan of `batch` interleaved sequences of n points
@@ -1165,9 +1210,10 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
     const size_t fixed = size_t(N) * cplx * (3 * R /*rinit*/ + 3 * 3 * R /*r*/ + 3 * R /*l*/ +
                                       3 * R /*J psi*/ + (c.sandwich ? 2 * 3 * R : 0));
     if (workspace == 0) {
-        size_t free_b = 0, total_b = 0;
+        size_t free_b = 0, total_b = 0, kept = 0;
         RSATB_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-        workspace = (free_b + ctx->work_bytes) / 10 * 8;  // the kept block is reused
+        RSATB_TRY(kept_work(ctx, &kept));  // this call takes it or gives it back
+        workspace = (free_b + kept) / 10 * 8;
     }
     // One launch per moment (moment_kernel) where the four matrices allow it
     // and its buffers (two panels, the start, the packed values) are no larger
@@ -1179,7 +1225,6 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
     FftchebSizes sizes{workspace, fixed,      nb, b, R, M, cplx, bastin,
                        part_bytes, ctx->sm_count * 2, sections};
     FftchebPartition part{};
-    T* wgt = nullptr;  // in the context's scratch
     const int64_t nnz = c.op->H->nnz_blocks;
     const size_t fixed_m =
         size_t(N) * cplx * 3 * 4 * R + 4 * size_t(nnz) * sizeof(T) + sizeof(int) + 256;
@@ -1192,17 +1237,14 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
     }
     if (one_launch) {
         void* sc = nullptr;
-        RSATB_TRY(ctx_scratch(ctx, 4 * size_t(nnz) * sizeof(T) + 256, &sc));
-        wgt = static_cast<T*>(sc);
-        int* d_differs = reinterpret_cast<int*>(wgt + 4 * nnz);
+        RSATB_TRY(ctx_scratch(ctx, sizeof(int), &sc));
+        int* d_differs = static_cast<int*>(sc);
         RSATB_CUDA_TRY(cudaMemsetAsync(d_differs, 0, sizeof(int), st));
         const rsatb_bsr_matrix* H = c.op->H;
-        pack_weights_kernel<T><<<grid_for(std::max<int64_t>(nnz, N + 1), ctx->sm_count), 256, 0,
-                                 st>>>(
-            N, nnz, H->row_ptr, H->col_ind, static_cast<const T*>(H->values), V[0]->row_ptr,
-            V[0]->col_ind, static_cast<const T*>(V[0]->values), V[1]->row_ptr, V[1]->col_ind,
-            static_cast<const T*>(V[1]->values), V[2]->row_ptr, V[2]->col_ind,
-            static_cast<const T*>(V[2]->values), wgt, d_differs);
+        compare_patterns_kernel<<<grid_for(std::max<int64_t>(nnz, N + 1), ctx->sm_count), 256, 0,
+                                  st>>>(N, nnz, H->row_ptr, H->col_ind, V[0]->row_ptr,
+                                        V[0]->col_ind, V[1]->row_ptr, V[1]->col_ind,
+                                        V[2]->row_ptr, V[2]->col_ind, d_differs);
         RSATB_LAUNCH_CHECK(ctx);
         int differs = 0;
         RSATB_CUDA_TRY(cudaMemcpyAsync(&differs, d_differs, sizeof(int), cudaMemcpyDeviceToHost,
@@ -1237,6 +1279,7 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
     const size_t e_bytes = part.e_bytes;
     const size_t oPan = one_launch ? mem.reserve(2 * panel * sizeof(T)) : 0;
     const size_t oInit = one_launch ? mem.reserve(panel * sizeof(T)) : 0;
+    const size_t oWgt = one_launch ? mem.reserve(4 * size_t(nnz) * sizeof(T)) : 0;
     const size_t oJ = one_launch ? 0 : mem.reserve(3 * v1);
     const size_t oRinit = one_launch ? 0 : mem.reserve(3 * v1);
     const size_t oR = one_launch ? 0 : mem.reserve(9 * v1);
@@ -1353,6 +1396,12 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
         ma.n_rows = N;
         ma.row_ptr = c.op->H->row_ptr;
         ma.col_ind = c.op->H->col_ind;
+        const rsatb_bsr_matrix* H = c.op->H;
+        T* const wgt = mem.at<T>(oWgt);
+        pack_weights_kernel<T><<<grid_for(nnz, ctx->sm_count), 256, 0, st>>>(
+            nnz, static_cast<const T*>(H->values), static_cast<const T*>(V[0]->values),
+            static_cast<const T*>(V[1]->values), static_cast<const T*>(V[2]->values), wgt);
+        RSATB_LAUNCH_CHECK(ctx);
         ma.wgt = wgt;
         ma.W1 = W1;
         ma.C = moment_threads_per_row<T>(R);

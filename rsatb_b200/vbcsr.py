@@ -75,6 +75,10 @@ class Context:
     def synchronize(self) -> None:
         check(lib().rsatb_ctx_synchronize(self.handle))
 
+    def release_workspace(self) -> None:
+        """Gives back the device memory that transport calls keep for the next one."""
+        check(lib().rsatb_ctx_release_workspace(self.handle))
+
     def launch_count(self) -> int:
         return int(lib().rsatb_ctx_launch_count(self.handle))
 

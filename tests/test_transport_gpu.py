@@ -390,3 +390,37 @@ def test_a_workspace_that_holds_the_separate_launches_is_accepted(torch_cuda):
     sig, _, st = _gpu(**kw, max_workspace_mb=ws / (1 << 20))
     assert st["sections"] == n
     assert rel_err(sig, _gpu(**kw)[0]) < 1e-12
+
+
+@pytest.mark.parametrize("M,bastin", [(512, False), (300, False), (300, True)])
+def test_kept_workspace_is_given_back(torch_cuda, M, bastin):
+    """What a call leaves with its context is memory that another allocator of the
+    process (torch's) can have: one allocation of what was free before the call."""
+    torch = torch_cuda
+    H, V = _tbg(m=5, tiles=(4, 4))
+    psi = _phases(H.n_rows, 8)
+    kw = dict(formulation=1) if bastin else {}
+    args = (torch, H, V, psi, M, -12.0, 12.0)
+    _gpu(*args, **kw)
+    torch.cuda.synchronize()
+    from rsatb_b200.vbcsr import context
+    context().release_workspace()
+    torch.cuda.empty_cache()
+    before = torch.cuda.mem_get_info()[0]
+    first = _gpu(*args, **kw)[0]
+    for _ in range(2):  # the second call in a row of one size starts to keep
+        sig, _, st = _gpu(*args, **kw)
+        assert np.array_equal(sig, first)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    assert st["store_bytes"] > 256 << 20
+    assert torch.cuda.mem_get_info()[0] < before - (128 << 20)
+    x = torch.empty(before - (128 << 20), dtype=torch.uint8, device="cuda")
+    del x
+    torch.cuda.empty_cache()
+    # and by the call that asks for it
+    for _ in range(2):
+        assert np.array_equal(_gpu(*args, **kw)[0], first)
+    torch.cuda.empty_cache()
+    context().release_workspace()
+    assert torch.cuda.mem_get_info()[0] >= before - (32 << 20)
