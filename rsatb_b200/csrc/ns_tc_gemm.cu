@@ -36,26 +36,6 @@ __device__ __forceinline__ void record_error(unsigned* error, unsigned code) {
     if (error) atomicOr(error, code);
 }
 
-// Stores one thread's 16 consecutive values of C (row `row`, columns col0..
-// col0 + 15 of the padded problem): the hi/lo pair and the optional FP64
-// copy at (row, col), and the optional transposed hi/lo at (col, row); with
-// args.sym only the upper triangle (col >= row) is stored, each element
-// also at (col, row), so C leaves exactly symmetric.  The transposed and
-// mirrored stores of a warp (32 consecutive rows, one column) are
-// coalesced; a warp's rows are a whole 32 of the padded problem, so the row
-// stores are formed by the warp together (store_rows_warp).
-// X (hi + lo) at (row, col0 .. col0 + 15) for the polynomial epilogue, read as
-// (col, row): X is symmetric up to rounding, and for a fixed column a warp's 32
-// rows are one 128-byte line (16 bytes a row, 32 lines an instruction, the other
-// way).
-__device__ __forceinline__ void load_x16(const TcArgs& args, const Prob& pr, int row, int col0,
-                                         float (&xe)[16]) {
-    const int64_t base = pr.off + int64_t(col0) * pr.n_pad + row;
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-        xe[j] = args.xe_hi[base + j * pr.n_pad] + args.xe_lo[base + j * pr.n_pad];
-}
-
 // 4 x 4 transpose of 16-byte quads over groups of four lanes: in, lane i holds
 // quads 0..3 of its row; out, quad i of the group's rows 0..3.
 __device__ __forceinline__ void quad_transpose(float (&v)[16], int lane) {
@@ -75,6 +55,28 @@ __device__ __forceinline__ void quad_transpose(float (&v)[16], int lane) {
             }
         }
     }
+}
+
+// X (hi + lo) at (row, col0 .. col0 + 15) for the polynomial epilogue: four lanes
+// read 64 contiguous bytes of each of their four rows, as store_rows_warp writes
+// them.  (Read as (col, row), a line per instruction too, the results are further
+// from the exact ones, 3.41e-5 against 3.35e-5 of 1,500 ragged problems: X is
+// symmetric up to rounding only.)
+__device__ __forceinline__ void load_x16(const TcArgs& args, const Prob& pr, int row, int col0,
+                                         float (&xe)[16]) {
+    const int lane = threadIdx.x & 31;
+    const int64_t base =
+        pr.off + int64_t(row - (lane & 3)) * pr.n_pad + col0 + 4 * (lane & 3);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float4 h = *reinterpret_cast<const float4*>(args.xe_hi + base + j * pr.n_pad);
+        const float4 l = *reinterpret_cast<const float4*>(args.xe_lo + base + j * pr.n_pad);
+        xe[4 * j] = h.x + l.x;
+        xe[4 * j + 1] = h.y + l.y;
+        xe[4 * j + 2] = h.z + l.z;
+        xe[4 * j + 3] = h.w + l.w;
+    }
+    quad_transpose(xe, lane);
 }
 
 // The 16 consecutive columns of a warp's 32 rows (row: this lane's), 64
@@ -111,6 +113,14 @@ __device__ __forceinline__ void store_rows(const TcArgs& args, int64_t base,
     }
 }
 
+// Stores one thread's 16 consecutive values of C (row `row`, columns col0..
+// col0 + 15 of the padded problem): the hi/lo pair and the optional FP64
+// copy at (row, col), and the optional transposed hi/lo at (col, row); with
+// args.sym only the upper triangle (col >= row) is stored, each element
+// also at (col, row), so C leaves exactly symmetric.  The transposed and
+// mirrored stores of a warp (32 consecutive rows, one column) are
+// coalesced; a warp's rows are a whole 32 of the padded problem, so the row
+// stores are formed by the warp together (store_rows_warp).
 __device__ __forceinline__ void store_chunk(const TcArgs& args, const Prob& pr, int row, int col0,
                                             float (&hi)[16], float (&lo)[16]) {
     const int np = pr.n_pad;
@@ -272,7 +282,9 @@ __global__ void __launch_bounds__(128, 1)
 
         // ---- epilogue, all 128 threads
         __syncwarp();
-        const bool ok = mbar_wait(&done, n_done & 1u, kWaitLimitNs);
+        // One answer per warp: the epilogue's TMEM loads and shuffles take all of it.
+        const bool ok =
+            __all_sync(0xffffffffu, mbar_wait(&done, n_done & 1u, kWaitLimitNs));
         ++n_done;
         if (!ok) {
             if (lane == 0) record_error(args.error, 4u);
@@ -556,7 +568,8 @@ __global__ void __launch_bounds__(320, 1)
             const Prob pr = cur.pr;
             const uint32_t b = t & 1u, tph = (t >> 1) & 1u;
             ++t;
-            if (!mbar_wait(&acc_full[b], tph, kWaitLimitNs)) {
+            // One answer per warp, as above.
+            if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[b], tph, kWaitLimitNs))) {
                 if (lane == 0) record_error(args.error, 4u);
                 abort_flag = 1;
                 break;
