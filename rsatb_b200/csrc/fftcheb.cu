@@ -1408,13 +1408,17 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
         ma.c = c.op->center;
         ma.inv_hw = 1.0 / c.op->half_width;
         ma.cscale = -1.0 / (2.0 * c.op->half_width);
-        // Rows per CTA: up to 256 threads, and as many as fit one pass of
-        // kMomentCap nonzeros.
+        // Rows per CTA: up to 256 threads, and as many average rows as fit one
+        // pass of kMomentCap nonzeros; a CTA with longer ones takes more passes.
+        // (By the longest row, one long row made every CTA a single row: 100,000
+        // rows of 9 nonzeros and one of 1,009, 4 FP64 samples 237 us a moment, now
+        // 103; the separate launches 1,177.)
         const int longest = std::max(1, c.op->H->max_row_blocks);
-        int rpc = std::min(256 / ma.C, kMomentCap / longest);
+        const int average = int(std::max<int64_t>(1, (nnz + N - 1) / std::max<int64_t>(N, 1)));
+        int rpc = std::min(256 / ma.C, kMomentCap / average);
         if (rpc < 1) rpc = 1;
         m_threads = rpc * ma.C;
-        ma.cap = std::min(kMomentCap, rpc * longest);
+        ma.cap = int(std::min<int64_t>(kMomentCap, int64_t(rpc) * longest));
         m_smem = size_t(ma.cap) * (4 * sizeof(T) + sizeof(int32_t));
         moment_init_kernel<T><<<grid_for(N * R, ctx->sm_count), 256, 0, st>>>(
             N, R, ma.row_ptr, ma.col_ind, ma.wgt, psi, ma.cscale, start);
