@@ -9,8 +9,10 @@
 #include "cheb_narrow.cuh"
 #include "cheb_dmma.cuh"
 #include "cheb_tf32.cuh"
+#include "dmma_any_rule.cuh"
 #include "step_launch.cuh"
 
+#include <algorithm>
 #include <cstdlib>
 
 namespace rsatb_b200 {
@@ -39,8 +41,12 @@ int launch(rsatb_context* ctx, Kernel kernel, int V, int64_t rows, StepArgs& a) 
     return RSATB_SUCCESS;
 }
 
+// Threads per SM (of 2,048 places) below which a launch leaves SMs idle.
+constexpr int kFewThreads = 440;
+
 // Picks V (values per thread) for W real values per row.
-inline int pick_v(int W, bool cv, bool any_b, int block_size, bool dbl, int64_t rows) {
+inline int pick_v(int W, bool cv, bool any_b, int block_size, bool dbl, int64_t rows,
+                  int sm_count) {
     const int forced = env_v();
     auto ok = [&](int v) {
         if (v <= 0 || W % v) return false;
@@ -60,7 +66,11 @@ inline int pick_v(int W, bool cv, bool any_b, int block_size, bool dbl, int64_t 
     (void)dbl;
     // Blocks with too few threads at 4 values each to fill the SMs take 2 (4,096
     // block rows of 5 x 5, real W = 32: FP32 27 -> 20 us a step; even from W = 64).
-    if (!cv && block_size > 1 && rows * W / 4 < 65536 && ok(2)) return 2;
+    // Only where W / 2 threads a row tile warps: FP32 blocks of 8 at W = 48 on 1,024
+    // block rows 22.8 us with 4 each, 26.9 with 2.
+    if (!cv && block_size > 1 && rows * W / 4 < int64_t(sm_count) * kFewThreads && ok(2) &&
+        (32 % (W / 2) == 0 || W / 2 % 32 == 0))
+        return 2;
     if (block_size == 1) {
         // Scalar rows: the first width whose W / V threads per row tile a
         // warp exactly (measured on the twisted-bilayer transport panel,
@@ -204,7 +214,7 @@ int launch_staged_v(rsatb_context* ctx, int V, StepArgs& a) {
 
 // V for the staged kernel: FP64 blocks of 8 take 2 values per thread (the
 // register tile stays near 100 registers), everything else 4 when it fits.
-inline int pick_v_staged(int W, bool cv, int block_size, bool dbl, int64_t rows) {
+inline int pick_v_staged(int W, bool cv, int block_size, bool dbl, int64_t rows, int sm_count) {
     const int forced = env_v();
     auto ok = [&](int v) {
         if (v <= 0 || v > 6 || W % v) return false;
@@ -213,8 +223,11 @@ inline int pick_v_staged(int W, bool cv, int block_size, bool dbl, int64_t rows)
         return (L <= 32 && 32 % L == 0) || (L > 32 && L % 32 == 0 && L <= 256);
     };
     if (forced && ok(forced)) return forced;
-    // As pick_v's: FP64 5 x 5 real W = 32 on 4,096 block rows 29.8 -> 28.0 us.
-    if (!cv && block_size > 1 && rows * W / 4 < 65536 && ok(2)) return 2;
+    // As pick_v's: FP64 5 x 5 real W = 32 on 4,096 block rows 29.8 -> 28.0 us.  Not
+    // beyond a warp per row: W = 128 on 512 and 1,024 block rows, a step with its
+    // dots 24 -> 48 and 36 -> 64 us.
+    if (!cv && block_size > 1 && W <= 64 && rows * W / 4 < int64_t(sm_count) * kFewThreads && ok(2))
+        return 2;
     const int real64[3] = {2, 4, 1}, real32[3] = {4, 2, 1}, cplx[3] = {4, 2, 6},
               cplx64[3] = {2, 4, 6};
     const int* pref = cv ? ((dbl && block_size == 8) ? cplx64 : cplx)
@@ -493,32 +506,11 @@ int launch_b(rsatb_context* ctx, int V, int64_t rows, StepArgs& a) {
     return set_error(RSATB_NOT_SUPPORTED, "no step kernel for V=%d", V);
 }
 
-// Where the any-shape tensor-core kernel is the default, measured on 4,096 block
-// rows of 17 blocks of 5 and 29 blocks of 8 (us per step of the doubled
-// recurrence, or per Y = A X where marked *; it against the best of the others).
-// W = 8, 16, 32, 64, 128 and 256 on blocks of 8 in FP64 (W <= 16 in FP32) stay
-// with the tiled tensor-core kernel before it, equal or faster.
-//   FP64 b = 8     every width: 7* 13 / 66, 24* 25 / 68, 45 78 / 218, 57* 67 / 188
-//   FP64 b < 8     b = 5: 8 18 / 34, 16 25 / 26, 24* 16 / 24, 45* 31 / 39, 57*
-//                  35 / 43; behind at multiples of 4 from 32 (33 / 30, 64 59 / 38)
-//   FP64 complex   b = 5, 6 columns 28 / 37, 16 35 / 34, 24 45 / 53; 32* 43 / 40,
-//                  64* 76 / 70, but 45* 60 / 62 and 57* 76 / 88, where the others
-//                  lose their wide loads
-//   FP32 b = 8     W < 64 off the bulk-copy widths: 7 20 / 38, 24 32 / 40, 45 60 /
-//                  81; complex panels of W = 90* 73 / 62
-//   FP32 b < 8     W <= 24: 7* 8.6 / 13.5, 16* 11 / 17, 24* 15 / 17; 32* 16 / 15
-//   FP32 complex   W <= 16: 6 columns 24 / 32, 8 24 / 31; 11* 29 / 21
-inline bool dmma_any_wanted(int W, int b, bool cm, bool dbl) {
-    if (dbl) return cm ? W <= 48 || W % 8 != 0 : b == 8 || W < 32 || W % 4 != 0;
-    if (cm) return W <= 16;
-    if (b != 8) return W <= 24;
-    return W < 64 && W != 32;
-}
-
 template <typename VT, typename MT, bool CM, bool CV>
-int launch_typed(rsatb_context* ctx, int block_size, StepArgs& a) {
+int launch_typed(rsatb_context* ctx, int block_size, double row_blocks, StepArgs& a) {
     const bool special = block_size == 1 || block_size == 5 || block_size == 8;
-    const int V = pick_v(a.W, CV, !special, block_size, sizeof(VT) == 8, a.n_block_rows);
+    const int V = pick_v(a.W, CV, !special, block_size, sizeof(VT) == 8, a.n_block_rows,
+                         ctx->sm_count);
     if (V == 0)
         return set_error(RSATB_NOT_SUPPORTED,
                          "panel width %d (real values per row) has no thread mapping; widths up "
@@ -542,7 +534,9 @@ int launch_typed(rsatb_context* ctx, int block_size, StepArgs& a) {
             if (st != kNotApplicable) return st;
         }
     }
-    if (forced == 9 || (forced == 0 && dmma_any_wanted(a.W, block_size, CM, sizeof(VT) == 8))) {
+    if (forced == 9 ||
+        (forced == 0 && dmma_any_wanted(a.W, block_size, CM, sizeof(VT) == 8, rows, row_blocks,
+                                        ctx->sm_count))) {
         const int st = launch_dmma_any<VT, CM, CV>(ctx, a);
         if (st != kNotApplicable) return st;
     }
@@ -566,7 +560,7 @@ int launch_typed(rsatb_context* ctx, int block_size, StepArgs& a) {
         // block rows are two per SM or more (4,096 rows, Y = A X: W = 32 39 us
         // against the register kernel's 25, W = 64 43 against 37; 32,768 rows,
         // W = 32 152 us).
-        const bool wide = a.W >= 32 && a.n_block_rows * a.W >= int64_t(296) * 1024;
+        const bool wide = a.W >= 32 && a.n_block_rows * a.W >= int64_t(ctx->sm_count) * 2 * 1024;
         if (block_size == 8 && (forced == 4 || (forced == 0 && wide))) {
             const int st = launch_bulk<CV>(ctx, a);
             if (st != kNotApplicable) return st;
@@ -583,7 +577,8 @@ int launch_typed(rsatb_context* ctx, int block_size, StepArgs& a) {
         forced == 2 ||
         (forced == 0 && block_size != 1 && (sizeof(VT) == 8 || (a.W == 16 && CV)));
     if (special && want_staged) {
-        const int Vs = pick_v_staged(a.W, CV, block_size, sizeof(VT) == 8, a.n_block_rows);
+        const int Vs = pick_v_staged(a.W, CV, block_size, sizeof(VT) == 8, a.n_block_rows,
+                                     ctx->sm_count);
         int st = kNotApplicable;
         if (Vs) {
             switch (block_size) {
@@ -622,15 +617,18 @@ int launch_step_precision(rsatb_context* ctx, const rsatb_bsr_matrix* A, int vec
     a.col_ind = A->col_ind;
     a.vals = A->values;
     a.block_size = A->block_size;
-    if (cm) return launch_typed<VT, VT, true, true>(ctx, A->block_size, a);
-    if (cv) return launch_typed<VT, VT, false, true>(ctx, A->block_size, a);
-    return launch_typed<VT, VT, false, false>(ctx, A->block_size, a);
+    // Average blocks of a row (a view of some rows carries the whole matrix's count).
+    const double row_blocks = std::min(double(A->max_row_blocks),
+                                       double(A->nnz_blocks) / std::max(1, A->n_block_rows));
+    if (cm) return launch_typed<VT, VT, true, true>(ctx, A->block_size, row_blocks, a);
+    if (cv) return launch_typed<VT, VT, false, true>(ctx, A->block_size, row_blocks, a);
+    return launch_typed<VT, VT, false, false>(ctx, A->block_size, row_blocks, a);
 }
 
 template <typename VT>
 int launch_coldot_precision(rsatb_context* ctx, int vec_dtype, int64_t n_rows, StepArgs& a) {
     const bool cv = dtype_is_complex(vec_dtype);
-    const int V = pick_v(a.W, cv, false, 1, sizeof(VT) == 8, n_rows);
+    const int V = pick_v(a.W, cv, false, 1, sizeof(VT) == 8, n_rows, ctx->sm_count);
     if (V == 0) return set_error(RSATB_NOT_SUPPORTED, "panel width %d not supported", a.W);
     a.dot_mode = DOT_PLAIN;
     a.n_block_rows = n_rows;
