@@ -146,8 +146,8 @@ __device__ __forceinline__ void fma_row(VT (&acc)[V], VT a, const VT (&x)[V]) {
     }
 }
 
-// ax += c y for V values of one row, rounded as the separate launch rounds
-// (the start c0 x too); a real panel takes Re(c).
+// ax += c y for V values of one row in FP64, rounded once a term as the separate
+// launch rounds (the start c0 x too); a real panel takes Re(c).
 template <typename VT, int V, bool CV>
 __device__ __forceinline__ void add_ax(const StepArgs& a, int64_t off, const VT (&xv)[V],
                                        const VT (&yv)[V]) {
@@ -289,8 +289,10 @@ __device__ __forceinline__ void finish_row(const StepArgs& a, int64_t row, int g
 // dst[o] = sum of n partial vectors of O values at P, P + step, ... (elements):
 // T = blockDim / O threads share an output where there are more threads than
 // outputs, their sums combined in part order; otherwise each thread takes whole
-// outputs.  Sixteen loads in flight per thread; a fixed order.  dst may be the
-// first vector.  All the CTA's threads (at most 256) call it.
+// outputs.  NL loads in flight per thread (sixteen cost most kernels registers and
+// with them CTAs per SM); a fixed order.  dst may be the first vector.  All the
+// CTA's threads (at most 256) call it.
+template <int NL = 8>
 __device__ __forceinline__ void sum_partials(const double* P, int n, size_t step, int O,
                                              double* dst) {
     __shared__ double comb[256];
@@ -300,13 +302,13 @@ __device__ __forceinline__ void sum_partials(const double* P, int n, size_t step
     for (int o = T > 1 ? threadIdx.x % O : threadIdx.x; o < O; o += T > 1 ? O : nt) {
         double sum = 0.0;
         if (part < T)
-            for (int b = part; b < n; b += 16 * T) {
-                double v[16];
+            for (int b = part; b < n; b += NL * T) {
+                double v[NL];
 #pragma unroll
-                for (int u = 0; u < 16; ++u)
+                for (int u = 0; u < NL; ++u)
                     v[u] = b + u * T < n ? __ldcg(P + size_t(b + u * T) * step + o) : 0.0;
 #pragma unroll
-                for (int h = 8; h > 0; h >>= 1)
+                for (int h = NL / 2; h > 0; h >>= 1)
 #pragma unroll
                     for (int u = 0; u < h; ++u) v[u] += v[u + h];
                 sum += v[0];
@@ -327,16 +329,20 @@ __device__ __forceinline__ void sum_partials(const double* P, int n, size_t step
 }
 
 // After every CTA wrote its partial dots: the last CTA to arrive (ticket
-// counters) sums them over the CTAs.  In two levels above 32 CTAs: the last of
-// every 32 sums its group's partials in place of the group's first, the last of
-// those sums the groups.  The sums sit on the step's critical path as a chain of
-// L2 round trips: at 1,024 CTAs of 24 outputs the step takes 34 us with one level
-// and four loads in flight, 30 with sixteen, 24 with both levels (17 without
-// dots); FP64 blocks of 8 at W = 32 58.9 -> 47.7, W = 16 38.0 -> 30.0.  The order is fixed for a given grid: deterministic dots.  Resets the
-// counters for the next launch.  Needs blockDim.x <= 256.
+// counters) sums them over the CTAs.  In two levels where a thread of that CTA
+// would have more than two rounds of loads (kOneLevel): the last of every 32 CTAs
+// sums its group's partials in place of the group's first, the last of those sums
+// the groups.  The sums sit on the step's critical path as a chain of L2 round
+// trips: at 1,024 CTAs of 24 outputs the step takes 34 us with one level, 24 with
+// both (17 without dots); FP64 blocks of 8 at W = 32 58.9 -> 47.7, W = 16 38.0 ->
+// 30.0; but at 128 CTAs of 16 outputs 8.7 us with one level and 10.4 with two.  The
+// order is fixed for a given grid: deterministic dots.  Resets the counters for the
+// next launch.  Needs blockDim.x <= 256.
 constexpr int kGroupCtas = 32;
+constexpr int kOneLevel = 16;       // values a thread sums alone at most
 constexpr int kGroupCounter0 = 8;   // the groups' counters: counter[8 + group]
 constexpr int kMaxGroups = 48;      // the fault word lies beyond them
+template <int NL = 8, int ONE = kOneLevel>
 __device__ __forceinline__ void finish_partials(const StepArgs& a, int ndots) {
     __threadfence();
     __syncthreads();
@@ -346,7 +352,7 @@ __device__ __forceinline__ void finish_partials(const StepArgs& a, int ndots) {
     int n = G;
     size_t step = O;
     const int groups = (G + kGroupCtas - 1) / kGroupCtas;
-    if (groups > 1 && groups <= kMaxGroups) {
+    if ((ONE ? G * O > ONE * int(blockDim.x) : groups > 1) && groups <= kMaxGroups) {
         const int group = blockIdx.x / kGroupCtas;
         const int size = min(kGroupCtas, G - group * kGroupCtas);
         unsigned* gc = a.counter + kGroupCounter0 + group;
@@ -356,7 +362,7 @@ __device__ __forceinline__ void finish_partials(const StepArgs& a, int ndots) {
         __threadfence();
         if (threadIdx.x == 0) *gc = 0u;
         double* P = a.partials + size_t(group) * kGroupCtas * O;
-        sum_partials(P, size, O, O, P);
+        sum_partials<NL>(P, size, O, O, P);
         n = groups;
         step = size_t(kGroupCtas) * O;
         __threadfence();
@@ -366,7 +372,7 @@ __device__ __forceinline__ void finish_partials(const StepArgs& a, int ndots) {
     __syncthreads();
     if (ticket != unsigned(n - 1)) return;
     __threadfence();
-    sum_partials(a.partials, n, step, O, a.dots_out);
+    sum_partials<NL>(a.partials, n, step, O, a.dots_out);
     if (threadIdx.x == 0) *a.counter = 0u;  // ready for the next launch
 }
 
@@ -396,10 +402,26 @@ __device__ __forceinline__ void reduce_dots(const StepArgs& a, int L, const doub
     finish_partials(a, ndots);
 }
 
+// CTAs per SM that the register kernel is compiled for (0: the compiler's choice).
+// Without it a few registers more or less, from any code after the main loop, move
+// the occupancy: scalar rows at 33 nonzeros and FP32 blocks of 8 went from 219 to
+// 357 us and from 102 to 153 us an application that way.
+template <typename VT, int B, int V, int AX>
+constexpr int step_min_ctas() {
+    constexpr bool d = sizeof(VT) == 8;
+    if (AX == 2) return 3;
+    if (B == 1) return V == 1 ? (d ? 6 : 5) : V == 2 ? 5 : V == 4 ? (d ? 4 : 0) : d ? 3 : 4;
+    if (B == 5) return V == 1 ? 5 : V == 2 ? 4 : V == 4 ? (d ? 2 : 3) : d ? 1 : 2;
+    return V == 1 ? 4 : V == 2 ? (d ? 2 : 3) : V == 4 ? (d ? 1 : 2) : 1;
+}
+
 // Compile-time block size B.  MT: real component type of the matrix values;
-// CM: complex matrix values; CV: complex panel.
-template <typename VT, typename MT, int B, int V, bool CM, bool CV>
-__global__ void __launch_bounds__(256) cheb_step_kernel(StepArgs a) {
+// CM: complex matrix values; CV: complex panel; AX (scalar rows): 1 adds into
+// StepArgs::ax, 2 reads x, p and four nonzeros ahead too.
+template <typename VT, typename MT, int B, int V, bool CM, bool CV, int AX = 0>
+__global__ void __launch_bounds__(256, step_min_ctas<VT, B, V, AX>())
+    cheb_step_kernel(StepArgs a) {
+    static_assert(!AX || B == 1, "the sum is added at scalar rows");
     static_assert(!CM || CV, "a complex matrix needs a complex panel");
     static_assert(!CV || V % 2 == 0, "complex panels need (re, im) pairs per thread");
     const int L = a.W / V;
@@ -422,8 +444,8 @@ __global__ void __launch_bounds__(256) cheb_step_kernel(StepArgs a) {
 #pragma unroll
             for (int v = 0; v < V; ++v) acc[r][v] = VT(0);
         const int k0 = __ldg(a.row_ptr + i), k1 = __ldg(a.row_ptr + i + 1);
-        if constexpr (B == 1 && !CM) {
-            // Scalar rows: x and p first, then four nonzeros in flight.
+        if constexpr (AX == 2) {
+            // x and p first, then four nonzeros in flight.
             const int64_t off = i * a.W + int64_t(g) * V;
             VT xv[V], pv[V];
 #pragma unroll
@@ -498,21 +520,23 @@ __global__ void __launch_bounds__(256) cheb_step_kernel(StepArgs a) {
         }
 #pragma unroll
         for (int r = 0; r < B; ++r)
-            finish_row<VT, V, CV, false, B == 1>(a, i * B + r, g, acc[r], d0, d1);
+            finish_row<VT, V, CV, false, AX != 0>(a, i * B + r, g, acc[r], d0, d1);
     }
     if (a.dot_mode != DOT_NONE) reduce_dots<V>(a, L, d0, d1);
 }
 
 // Whether a step on A adds into StepArgs::ax: the register kernel of scalar
 // rows does (its default), where the separate launch that reads the step's
-// output back was a third of a term (graphene, 80,000 rows x 4 FP64 complex
-// columns: 5.7 + 3.2 us in two launches, 7.6 in one).
+// output back was a third of a term (us a term in two launches and in one: 80,000
+// rows of 4 nonzeros, 4 FP64 complex columns 12.7, 10.3; 64 99.8, 83; 300,000 rows
+// of 33, 32 FP32 complex columns 268, 260).
 bool step_takes_ax(const rsatb_bsr_matrix* A);
 
 // Runtime block size (b <= 16): the fallback for block sizes without a
 // specialisation.  Same arithmetic, rows of the block handled one at a time.
 template <typename VT, typename MT, int V, bool CM, bool CV>
-__global__ void __launch_bounds__(256) cheb_step_kernel_any_b(StepArgs a) {
+__global__ void __launch_bounds__(256, sizeof(VT) == 8 && !CV ? 4 : 5)
+    cheb_step_kernel_any_b(StepArgs a) {
     const int L = a.W / V;
     const int g = threadIdx.x % L;
     const int B = a.block_size;

@@ -135,7 +135,9 @@ __device__ __forceinline__ void reduce_dots_staged(const StepArgs& a, int Lp, in
 }
 
 template <typename VT, typename MT, int B, int V, bool CM, bool CV, int STAGES>
-__global__ void __launch_bounds__(256) cheb_step_staged(StepArgs a, int Lp, int n_chunks) {
+// (The CTAs per SM are stated as step_min_ctas' are: 5 x 5 real W = 32 on 8,192
+// rows, FP64 49.6 us of a term at the compiler's choice, 43 so.)
+__global__ void __launch_bounds__(256, B == 5 && V == 4 ? 2 : 1) cheb_step_staged(StepArgs a, int Lp, int n_chunks) {
     static_assert(!CV || V % 2 == 0, "complex panels need (re, im) pairs per thread");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int RW = B * (CM ? 2 : 1);       // values per block row of A

@@ -492,7 +492,27 @@ template <typename VT, typename MT, int B, bool CM, bool CV>
 int launch_b(rsatb_context* ctx, int V, int64_t rows, StepArgs& a);
 
 template <typename VT, typename MT, int B, bool CM, bool CV>
-int launch_b(rsatb_context* ctx, int V, int64_t rows, StepArgs& a) {
+int launch_b(rsatb_context* ctx, int V, int64_t rows, double row_blocks, StepArgs& a) {
+    if constexpr (B == 1) {
+        if (a.ax) {
+            // Reading ahead pays for short rows and narrow FP64 panels that L2
+            // holds (4 nonzeros, us a term without and with it: 80,000 rows, 4
+            // complex columns 10.3, 8.3, 8 real ones 10.3, 9.0; 300,000 rows 22.4,
+            // 23.2 and 22.4, 23.4; 33 nonzeros, 64 real columns 642, 752).
+            if constexpr (sizeof(VT) == 8 && !CM) {
+                if (V == 4 && a.W <= 16 && row_blocks <= 5.0 && rows * a.W <= (int64_t(3) << 19))
+                    return launch(ctx, cheb_step_kernel<VT, MT, 1, 4, CM, CV, 2>, 4, rows, a);
+            }
+            if (V == 4) return launch(ctx, cheb_step_kernel<VT, MT, 1, 4, CM, CV, 1>, 4, rows, a);
+            if (V == 2) return launch(ctx, cheb_step_kernel<VT, MT, 1, 2, CM, CV, 1>, 2, rows, a);
+            if constexpr (CV) {
+                if (V == 6)
+                    return launch(ctx, cheb_step_kernel<VT, MT, 1, 6, CM, CV, 1>, 6, rows, a);
+            } else if (V == 1) {
+                return launch(ctx, cheb_step_kernel<VT, MT, 1, 1, CM, CV, 1>, 1, rows, a);
+            }
+        }
+    }
     switch (V) {
         case 1:
             if constexpr (!CV) return launch(ctx, cheb_step_kernel<VT, MT, B, 1, CM, CV>, 1, rows, a);
@@ -590,9 +610,9 @@ int launch_typed(rsatb_context* ctx, int block_size, double row_blocks, StepArgs
         if (st != kNotApplicable) return st;
     }
     switch (block_size) {
-        case 1: return launch_b<VT, MT, 1, CM, CV>(ctx, V, rows, a);
-        case 5: return launch_b<VT, MT, 5, CM, CV>(ctx, V, rows, a);
-        case 8: return launch_b<VT, MT, 8, CM, CV>(ctx, V, rows, a);
+        case 1: return launch_b<VT, MT, 1, CM, CV>(ctx, V, rows, row_blocks, a);
+        case 5: return launch_b<VT, MT, 5, CM, CV>(ctx, V, rows, row_blocks, a);
+        case 8: return launch_b<VT, MT, 8, CM, CV>(ctx, V, rows, row_blocks, a);
         default:
             if (V == 2) return launch(ctx, cheb_step_kernel_any_b<VT, MT, 2, CM, CV>, 2, rows, a);
             if constexpr (!CV)

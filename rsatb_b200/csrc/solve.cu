@@ -51,7 +51,7 @@ __device__ __forceinline__ double2 col_value(const double* d, int c) {
 // |rr_c|), and rr_out_c = <R_c|R_c> of the updated R: thread (sub, column)
 // of a CTA walks every (subs x gridDim.x)-th row, the CTA sums its rows in
 // a fixed order, and the CTA partials are summed as finish_partials sums them,
-// in two levels of 32 CTAs (kGroupCounter0).  Deterministic.  The last CTA also
+// in two levels of 32 CTAs where one is long (kOneLevel).  Deterministic.  The last CTA also
 // writes the residuals to host memory (pinned), which the host reads after the
 // event behind this launch: no copy between the iterations.
 // 32,768 rows x 16 FP64 columns: 10.6 us with four CTAs per SM (eight 13.9; two
@@ -112,7 +112,7 @@ cg_update_kernel(T* __restrict__ X, const T* __restrict__ P, T* __restrict__ R,
     int n = int(gridDim.x);
     size_t step = ncols;
     const int groups = (n + kGroupCtas - 1) / kGroupCtas;
-    if (groups > 1 && groups <= kMaxGroups) {
+    if (n * ncols > kOneLevel * kDotThreads && groups <= kMaxGroups) {
         const int group = blockIdx.x / kGroupCtas;
         const int size = min(kGroupCtas, n - group * kGroupCtas);
         unsigned* gc = counter + kGroupCounter0 + group;
