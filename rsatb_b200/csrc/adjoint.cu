@@ -135,9 +135,12 @@ __global__ void __launch_bounds__(128) sddmm_dmma_kernel(int n_block_rows, int n
             const int n = min(col0 + 8 * u + fr, cols - 1), blk = n / b;
             Tr[u] = T + (int64_t(__ldg(col_ind + kb + blk)) * b + (n - blk * b)) * R;
         }
-        double acc[kSdTiles][2];
+        // Two sums a tile, of the even and the odd k': half the chain each (its
+        // length shows in the rounding).
+        double acc[2][kSdTiles][2];
 #pragma unroll
-        for (int u = 0; u < kSdTiles; ++u) acc[u][0] = acc[u][1] = 0.0;
+        for (int u = 0; u < kSdTiles; ++u)
+            acc[0][u][0] = acc[0][u][1] = acc[1][u][0] = acc[1][u][1] = 0.0;
         // (q, s) of this lane's two k'
         int q0 = 2 * fc / R, s0 = 2 * fc - q0 * R;
         int q1 = (2 * fc + 1) / R, s1 = 2 * fc + 1 - q1 * R;
@@ -166,8 +169,8 @@ __global__ void __launch_bounds__(128) sddmm_dmma_kernel(int n_block_rows, int n
             const double a1 = v1 ? (n0 + q1 ? 2.0 : 1.0) * double(l1) : 0.0;
 #pragma unroll
             for (int u = 0; u < kSdTiles; ++u) {
-                dmma_884(acc[u], a0, v0 ? double(t0[u]) : 0.0);
-                dmma_884(acc[u], a1, v1 ? double(t1[u]) : 0.0);
+                dmma_884(acc[0][u], a0, v0 ? double(t0[u]) : 0.0);
+                dmma_884(acc[1][u], a1, v1 ? double(t1[u]) : 0.0);
             }
             q0 += dq;
             s0 += ds;
@@ -190,7 +193,7 @@ __global__ void __launch_bounds__(128) sddmm_dmma_kernel(int n_block_rows, int n
                     const int n = col0 + 8 * u + 2 * fc + v, blk = n / b;
                     if (n < cols)
                         grad[(int64_t(kb + blk) * b + fr) * b + (n - blk * b)] +=
-                            scale * acc[u][v];
+                            scale * (acc[0][u][v] + acc[1][u][v]);
                 }
         }
     }
