@@ -566,10 +566,12 @@ inline int fused_radix(int M) {
 // Exchange entries of one sequence; pairs of sequences per CTA; partial sums.
 __host__ __device__ constexpr int fused_xch(int r) { return 16 * (16 * r + r); }
 __host__ __device__ constexpr int fused_pairs(int r) { return 8 / r; }
-// Shared memory: exchange, w^j (j < M / 4), ph.
+// Tables: w^j (j < M / 4), ph (M), and pass B's w^{16 n0 k1} at n0 * 17 + k1.
+__host__ __device__ constexpr int fused_tab(int r) { return 64 * r + 256 * r + 17 * r; }
+// Shared memory: exchange, tables.
 template <typename C>
 size_t fused_smem(int r) {
-    return size_t(2 * fused_pairs(r) * fused_xch(r) + 64 * r + 256 * r) * sizeof(C);
+    return size_t(2 * fused_pairs(r) * fused_xch(r) + fused_tab(r)) * sizeof(C);
 }
 
 // Complex arithmetic on float2 (FP32 transform) and double2 (FP64 transform).
@@ -713,7 +715,7 @@ __device__ __forceinline__ C load_c(const double* S, int64_t e) {
 // CTA's threads run it together (xch: this sequence's exchange buffer).
 template <typename C, int r, typename T>
 __device__ __forceinline__ void fused_transform(const T* S, int t, const C* qtw, const C* ph,
-                                                C* xch, C (&out)[16]) {
+                                                const C* wb, C* xch, C (&out)[16]) {
     constexpr int M = 256 * r, TPS = 16 * r;
     C v[16];
 #pragma unroll
@@ -739,10 +741,13 @@ __device__ __forceinline__ void fused_transform(const T* S, int t, const C* qtw,
     dft16_inv(v);
     __syncthreads();
     if constexpr (r > 1) {
-        const Pow16<C> tw(twiddle<C, M>(qtw, 16 * n0), twiddle<C, M>(qtw, 64 * n0));
+        // Read, not formed as powers: a pass-B factor multiplies 16 r outputs of the
+        // sequence alike, so its rounding adds up in the sums of products (FP32, 2048
+        // moments, 16 samples of 47,632 rows: sigma off by 1.50e-7 with powers).
+        xch[t] = v[dft16_at(0)];
 #pragma unroll
-        for (int k1 = 0; k1 < 16; ++k1)
-            xch[k1 * (16 * r + 1) + t] = c_mul(v[dft16_at(k1)], tw(k1));
+        for (int k1 = 1; k1 < 16; ++k1)
+            xch[k1 * (16 * r + 1) + t] = c_mul(v[dft16_at(k1)], wb[n0 * 17 + k1]);
     } else {
 #pragma unroll
         for (int k1 = 0; k1 < 16; ++k1) xch[k1 * (16 * r + 1) + t] = v[dft16_at(k1)];
@@ -761,7 +766,7 @@ __device__ __forceinline__ void fused_transform(const T* S, int t, const C* qtw,
     __syncthreads();  // xch is rewritten
 }
 
-// The tables of the transform: tab[j] = w^j (j < M / 4), tab[M / 4 + m] = ph_m.
+// The tables of the transform (fused_tab): w^j, ph_m and pass B's factors.
 __global__ void fused_tables_kernel(int M, const double* w, double2* tab) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     double s, c;
@@ -772,6 +777,10 @@ __global__ void fused_tables_kernel(int M, const double* w, double2* tab) {
         const int m = i - M / 4;
         sincospi(double(m) / (2.0 * double(M)), &s, &c);  // e^{i pi m / 2M}
         tab[i] = make_double2(w[m] * c, w[m] * s);
+    } else if (i < fused_tab(M / 256)) {
+        const int e = i - (M / 4 + M);  // w^{16 n0 k1} = e^{2 pi i n0 k1 / 16 r}
+        sincospi(double((e / 17) * (e % 17)) / (8.0 * double(M / 256)), &s, &c);
+        tab[i] = make_double2(c, s);
     }
 }
 
@@ -813,7 +822,8 @@ __global__ void __launch_bounds__(kFusedThreads, 2)
     C* xch0 = reinterpret_cast<C*>(fsm_raw);
     C* qtw = xch0 + 2 * P * fused_xch(r);
     C* ph = qtw + M / 4;
-    for (int j = threadIdx.x; j < M / 4 + M; j += blockDim.x)
+    C* wb = ph + M;
+    for (int j = threadIdx.x; j < fused_tab(r); j += blockDim.x)
         qtw[j] = Cx<C>::make(typename Cx<C>::S(tab[j].x), typename Cx<C>::S(tab[j].y));
     __syncthreads();
     const int seq = threadIdx.x / TPS, t = threadIdx.x - seq * TPS;
@@ -830,8 +840,8 @@ __global__ void __launch_bounds__(kFusedThreads, 2)
         const int64_t i = i0 + pair;
         const bool live = i < nqc;
         C out[16];
-        fused_transform<C, r>(Tq + 2 * (side * nqc + (live ? i : nqc - 1)) * M, t, qtw, ph, mine,
-                              out);
+        fused_transform<C, r>(Tq + 2 * (side * nqc + (live ? i : nqc - 1)) * M, t, qtw, ph, wb,
+                              mine, out);
         // The left thread gives its outputs 8.. and takes the right's 0..7.
 #pragma unroll
         for (int j = 0; j < 8; ++j)
@@ -1301,7 +1311,7 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
     const int fused_grid = part.ctas;
     const int n_part = fused ? fused_grid * fused_pairs(radix) : 0;
     const size_t oPart = fused ? mem.reserve(size_t(n_part) * M * sizeof(double2)) : 0;
-    const size_t oTab = fused ? mem.reserve(size_t(M / 4 + M) * sizeof(double2)) : 0;
+    const size_t oTab = fused ? mem.reserve(size_t(fused_tab(radix)) * sizeof(double2)) : 0;
     // cuFFT's work area, for the chunk sizes of a full section.
     const int fft_n = bastin ? 2 * M : M;
     size_t fft_work = 0;
@@ -1372,7 +1382,7 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
         if (c > 0 && c < fused_qc) fused_qc = c;
     }
     if (fused) {
-        fused_tables_kernel<<<(M / 4 + M + 255) / 256, 256, 0, st>>>(M, d_wts, d_tab);
+        fused_tables_kernel<<<(fused_tab(radix) + 255) / 256, 256, 0, st>>>(M, d_wts, d_tab);
         RSATB_LAUNCH_CHECK(ctx);
     }
 
