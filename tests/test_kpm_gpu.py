@@ -554,6 +554,39 @@ def test_propagate_matches_dense(torch_cuda, case):
     assert (Yd.cpu().numpy() == 3.0).all()
 
 
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+@pytest.mark.parametrize("R", [1, 3, 4, 40])
+@pytest.mark.parametrize("cm,cv", [(False, True), (False, False), (True, True)],
+                         ids=["complex_panel", "real_panel", "complex_rows"])
+def test_propagate_on_scalar_rows(torch_cuda, monkeypatch, cm, cv, R, precision):
+    """Scalar rows add every term in the step's epilogue: against the dense sum,
+    and as the launches that read the step's output back, bit for bit but for FP64
+    complex products, whose two roundings a term (2^-53 each) may fall either way."""
+    torch = torch_cuda
+    rng = np.random.default_rng(R)
+    H = random_hermitian_bsr(150, 1, 4, seed=R, complex_values=cm, scale=0.3)
+    b = np.abs(np.linalg.eigvalsh(H.to_dense())).max() + 0.5
+    X = _panel(rng, H.n_rows, R, cv)
+    dt = {("f64", True): torch.complex128, ("f64", False): torch.float64,
+          ("f32", True): torch.complex64, ("f32", False): torch.float32}[(precision, cv)]
+    c = build_cheby(H, -b, b, None, precision=precision)
+    Xd = to_dev(torch, X, dt)
+    for n in (1, 2, 3, 14):
+        coeffs = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+        Yd = torch.full_like(Xd, float("nan"))
+        c.propagate(Xd, Yd, coeffs)
+        want = _propagate_ref(_dense_op(H, -b, b, None), X, coeffs if cv else coeffs.real)
+        assert rel_err(Yd.cpu().numpy(), want) < (1e-13 if precision == "f64" else 1e-5)
+        monkeypatch.setenv("RSATB_STEP_KERNEL", "generic")
+        Zd = torch.full_like(Xd, float("nan"))
+        c.propagate(Xd, Zd, coeffs)
+        monkeypatch.delenv("RSATB_STEP_KERNEL")
+        if precision == "f64" and cv:
+            assert rel_err(Yd.cpu().numpy(), Zd.cpu().numpy()) <= 2 * n * 2.0 ** -53, n
+        else:
+            assert torch.equal(Yd, Zd), n
+
+
 def test_apply_dual_orthogonal_and_sandwich(torch_cuda):
     """Chebyshev::apply_dual: scale * V X (orthogonal) and scale * Z^H V Z X
     (sandwich) with an imaginary-unit velocity matrix."""

@@ -424,3 +424,58 @@ def test_kept_workspace_is_given_back(torch_cuda, M, bastin):
     torch.cuda.empty_cache()
     context().release_workspace()
     assert torch.cuda.mem_get_info()[0] >= before - (32 << 20)
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+@pytest.mark.parametrize("M", [256, 512, 1024, 2048])
+def test_fused_row_stage_at_every_radix(torch_cuda, precision, M, monkeypatch):
+    """303 sequences per axis (no whole number of a CTA's 8 / r pairs) through the
+    fused stage: against the cuFFT stage on the same stores and, in FP64, the
+    oracle; in chunks of 37, in one CTA's worth and in three sections."""
+    H, V = _scalar_chain(101, 9, seed=M)
+    psi = _phases(101, 3, seed=6)
+    args = (torch_cuda, H, V, psi, M, -8.0, 8.0, precision)
+    fused, en, st = _gpu(*args)
+    three, _, st3 = _gpu(*args, partition_sections=3)
+    for chunk in ("37", "1"):
+        monkeypatch.setenv("RSATB_FFTCHEB_CHUNK", chunk)
+        small, _, st_s = _gpu(*args)
+        assert st_s["fft_chunks"] == 3 * -(-303 // int(chunk))
+        assert rel_err(small, fused) < 1e-13
+    monkeypatch.delenv("RSATB_FFTCHEB_CHUNK")
+    monkeypatch.setenv("RSATB_FFTCHEB_FUSED", "0")
+    chunked, _, _ = _gpu(*args)
+    assert st["fft_chunks"] == 3 and st3["sections"] == 3
+    # FP64 transforms of the same stores but for FP32 vectors at 2048 moments: some
+    # twelve roundings of 6e-8 an output, twice in a product (1.4e-6), times what the
+    # 303 products of independent chains cancel to (their sum is about 1 / sqrt(303)
+    # of their absolute sum: 17, of which the roundings' own cancellation leaves 1
+    # to 4)
+    assert rel_err(fused, chunked) < (6e-6 if precision == "f32" and M == 2048 else 1e-12)
+    assert rel_err(three, fused) < 1e-12
+    if precision == "f64":
+        sig_o, en_o = _oracle(H, V, psi, M, -8.0, 8.0)
+        assert np.allclose(en, en_o, rtol=0, atol=1e-13)
+        assert rel_err(fused, sig_o) < 1e-10
+
+
+def test_kept_plans_and_workspaces_of_other_sizes(torch_cuda):
+    """More chunk sizes than plans are kept, workspaces that grow, shrink and
+    come back: every call's result is the one it gave alone."""
+    H, V = _tbg()
+    emin, emax = _bounds(H)
+    psi = _phases(H.n_rows, 2, seed=12)
+
+    def call(M, **kw):
+        return _gpu(torch_cuda, H, V, psi, M, emin, emax, **kw)[0]
+
+    kinds = [(40, {}), (50, dict(max_workspace_mb=8.0)), (60, dict(formulation=1)),
+             (50, dict(partition_sections=3)), (256, {})]
+    alone = []
+    for M, kw in kinds:
+        from rsatb_b200.vbcsr import context
+        context().release_workspace()
+        alone.append(call(M, **kw))
+    for k in (0, 1, 2, 3, 4, 0, 0, 1, 1, 2, 2, 0, 4, 4, 0, 3, 3, 2):
+        M, kw = kinds[k]
+        assert np.array_equal(call(M, **kw), alone[k]), k
