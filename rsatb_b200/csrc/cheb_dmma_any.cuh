@@ -19,7 +19,7 @@
 // for 69,632 blocks of 5; by the FP64 tensor pipe (26.6 TF/s measured for this
 // tile) at wide ones.  With the lane's offsets formed at every step and masked
 // loads these took 22.8 and 12.6 us, complex blocks of 5 at 6 columns 45 us
-// (now 16.8).  Against the kernels it replaces: dmma_any_wanted.
+// (now 16.8).  Against the kernels it replaces: dmma_any_rule.cuh.
 #pragma once
 
 #include "cheb_dmma.cuh"

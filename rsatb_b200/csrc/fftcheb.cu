@@ -25,7 +25,7 @@
 //   the same summation order on every run;
 // * at M = 256, 512, 1024 and 2048 (Greenwood) the row stage is one
 //   hand-written kernel after a coalesced gather: transform and contraction
-//   without the FP64 extension buffer's round trips (greenwood_fused_kernel).
+//   without a transform buffer's round trips (greenwood_fused_kernel).
 #include "cheb_kernels.cuh"
 #include "fftcheb_partition.cuh"
 
@@ -127,8 +127,8 @@ __global__ void store_right_vec_kernel(int64_t row0, int64_t rows, int R, const 
 // and indices are one contiguous run, staged in shared memory: read per thread
 // they were a serial chain of first touches (110 us per moment against 75.8 at
 // 47,632 rows of 33 nonzeros, 16 FP32 samples), and only the gathered rows are
-// left to wait for.  Bound by the latency of those (512 bytes per nonzero, 57 %
-// L1 hits), 32 warps x 4 loads per SM.  The six launches this replaces (left
+// left to wait for.  Bound by the latency of those (512 bytes per nonzero, 55 %
+// L1 hits at 11,908 rows), 32 warps x 4 loads per SM.  The six launches this replaces (left
 // step, right step, three currents, store copy) took 141 us; 11,536 rows x 5
 // FP64 samples: 18.7 us against 51.
 template <typename T>
@@ -401,7 +401,8 @@ __global__ void dct3_input_kernel(int M, int64_t nq, int chunk_rows, int R, int6
 
 // Bastin phi1 / phi2 inputs (fftcheb_transport.hpp:453-461, fft.hpp:156-174):
 // the weighted moments w[m] S_m (complex w) in the first M points of a
-// 2M-point sequence, zeros in the last M.  Layout as extend_kernel.
+// 2M-point sequence, zeros in the last M; [point][sequence], the sequences in
+// dct3_input_kernel's order.
 template <typename T>
 __global__ void pad_kernel(int M, int64_t nq, int chunk_rows, int R, int64_t sec_rows,
                            int64_t row_off, int64_t slot_elems, const T* S, const double2* w,
@@ -899,8 +900,7 @@ __global__ void __launch_bounds__(128) fused_reduce_kernel(int M, int n_part,
     K[2 * (int64_t(k) * 6 + comp) + 1] += red[0].y * inv;
 }
 
-// One chunk of the fused stage: grid CTAs (returned to the caller for sizing
-// through fused_grid) of the transform's type and radix.
+// One chunk of the fused stage, for the transform's type and radix.
 template <typename T, typename C, int r>
 int fused_launch(rsatb_context* ctx, int grid, int64_t n, const T* Tq, const double2* tab,
                  double2* partial) {
@@ -1302,7 +1302,7 @@ int fftcheb_impl(const Ctx& c, const rsatb_bsr_matrix* const* V, const T* psi, i
     const size_t oWts = mem.reserve(size_t(M) * sizeof(double));
     const size_t oPw = bastin ? mem.reserve(2 * size_t(M) * sizeof(double2)) : 0;
     // Fused row stage: up to two CTAs per SM, partial sums per CTA, pair of sequences
-    // and energy; chunks of fused_qc sequences gathered into the extension
+    // and energy; chunks of fused_qc sequences gathered into the transform
     // buffer (sequence-major, both sides).  FP32 vectors take the FP32
     // transform at M = 2048 (FP64 products and sums) unless
     // RSATB_FFTCHEB_FP64=1; every other case the FP64 one.

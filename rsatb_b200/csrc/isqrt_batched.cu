@@ -25,9 +25,10 @@
 // of its upper triangle only and mirrored, so it is exactly symmetric, and
 // a symmetric perturbation only moves Z normal to the solution set, which
 // the following steps undo.  Z' = P Z takes Z^T as its K-major B operand,
-// which the update itself stores (transposed) for the next step.  Each phase of a chunk is one captured
-// CUDA graph; a problem that stops early is gated off in every later kernel
-// by its `active` flag and its iterate is retired (copied out) at once.
+// which the update itself stores (transposed) for the next step.  A chunk's
+// iterations are launched one after the other and end with the last problem
+// still going (run_phase); a problem that stops early is gated off in every later
+// kernel by its `active` flag and its iterate is retired (copied out) at once.
 #include "ns_batched.cuh"
 #include "umma.cuh"
 
@@ -53,7 +54,6 @@ __device__ __forceinline__ void for_elements(int rows, int cols, F&& f) {
     for (int r = blockIdx.y * warps + (threadIdx.x >> 5); r < rows; r += gridDim.y * warps)
         for (int c = threadIdx.x & 31; c < cols; c += 32) f(r, c);
 }
-
 
 // S (row-major, padded, symmetric from the upper triangle of the
 // column-major input) in FP64 and, for a tensor-core phase, as TF32 hi/lo.
@@ -584,7 +584,8 @@ struct Dev {
     F64Item* f64_items_upper;  // the 64 x 64 tiles on or above the diagonal
     // live[k] (tensor-core phase) and live_f64[k] (FP64 phase): set by the
     // control step of iteration k when a problem goes on; the GEMMs after it
-    // return at once when it stays 0 (the graph keeps the full loop).
+    // return at once when it stays 0 (the host, which reads it one iteration
+    // behind, has the next iteration queued by then).
     int* live;
     int* live_f64;
     int n_live;
@@ -710,7 +711,7 @@ int run_chunk(rsatb_context* ctx, const Opts& o, const Chunk& ch, const int* col
     const int P = int(ch.probs.size());
     const bool low = o.precision != RSATB_NS_FP64;
     const bool split = o.precision == RSATB_NS_TF32X3;
-    // Dynamic shared-memory opt-in of the FP64 GEMMs, before any capture.
+    // Dynamic shared-memory opt-in of the FP64 GEMMs.
     RSATB_CUDA_TRY(cudaFuncSetAttribute(gemm_f64_kernel<true, false>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         int(F64Shape<true, false>::SMEM)));

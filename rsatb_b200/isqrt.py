@@ -55,7 +55,8 @@ def inverse_sqrt_columns_batched(M: torch.Tensor, n, in_offset, col_start=None, 
     p's n_p x k_p column-major block at out_offset[p] (packed in problem
     order when out_offset is None), status one rsatb_status per problem,
     stats a dict of the call's counters.  tiles: the tensor-core kernel and
-    N tiles picked by autotune_tiles (None: the built-in choice).
+    N tiles picked by autotune_tiles (None: the built-in choice).  graph is
+    accepted without effect: the iterations are launched directly.
     """
     if not (M.is_cuda and M.dtype == torch.float64 and M.dim() == 1 and M.is_contiguous()):
         raise ValueError("M must be a contiguous 1-D float64 CUDA tensor")

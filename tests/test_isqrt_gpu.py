@@ -154,6 +154,7 @@ def test_chain_diverging_healthy_capped(torch_cuda, precision):
 
 
 def test_graph_and_chunks_do_not_change_results(torch_cuda):
+    """Several chunks give the bits of one; graph is accepted without effect."""
     from rsatb_b200.isqrt import inverse_sqrt_columns_batched
     sizes = [48, 160, 96, 300, 33, 64]
     mats = _batch(sizes, [1e2, 1e4, 1e3, 1e5, 10.0, 1e5], seed=21)

@@ -272,8 +272,8 @@ def test_qe_route_sandwich_and_errors(torch_cuda):
 
 @pytest.mark.parametrize("precision", ["f64", "f32"])
 def test_fused_row_stage_at_2048_moments(torch_cuda, precision, monkeypatch):
-    """M = 2048 takes the fused Greenwood row stage (extension, 4096-point
-    DCT-III and contraction in one kernel): equal to the chunked cuFFT row
+    """M = 2048 takes the fused Greenwood row stage (the DCT-III as a 2048-point
+    transform, and the contraction, in one kernel): equal to the chunked cuFFT row
     stage on the same stores, over one section and three, and to the oracle.
     FP32 vectors take the FP32 transform (FP64 products and sums): within
     1e-6 of the FP64 transform of the same stores, which equals cuFFT's."""
