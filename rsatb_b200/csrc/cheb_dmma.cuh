@@ -52,11 +52,13 @@ struct DmmaShape {
 };
 
 // CTAs per SM, as step_min_ctas (0: the compiler's choice): FP64 complex panels of
-// 8 columns on 1,024 block rows 10.6 us at the compiler's choice, 8.3 so.
+// 8 columns on 1,024 block rows 10.6 us at the compiler's choice, 8.3 so.  Wider
+// panels spill where they are held to more CTAs: 128 columns on 32,768 block rows
+// 979 us at 4, 945 so; 64 on 4,096 79.2 at 6, 75.7 so.
 template <typename VT, int W, int UU>
 constexpr int dmma_min_ctas() {
     if (UU || sizeof(VT) == 4) return 0;
-    return W <= 32 ? 8 : W <= 64 ? 6 : W <= 128 ? 4 : 3;
+    return W <= 32 ? 8 : 0;
 }
 
 template <typename VT, int W, bool CV, int UU>
