@@ -103,10 +103,12 @@ __global__ void __launch_bounds__(256) sddmm_kernel(int n_block_rows, const int3
 // loaded once for all of them, and there is no reduction at the end.  Lane fc
 // takes k' = 8 t + 2 fc and + 1 for the two tiles of a step (the order of a sum's
 // terms is free), one 2-value load each when R is even.
-// Bound by the FP64 tensor pipe; 69,632 blocks of 5, 32 FP64 samples, a segment
-// of 16 moments: 213 us (261 with a tile per block, 891 with a warp per
+// Waits on its gathered panel rows with the FP64 tensor pipe half busy (47 %, L2
+// hits 75 %); 69,632 blocks of 5, 32 FP64 samples, a segment of 16 moments:
+// 205 us under the profiler (261 with a tile per block, 891 with a warp per
 // (block, row) and a shuffle tree).
 constexpr int kSdTiles = 6;
+constexpr int kSdFold = 4;  // 32 terms
 
 template <typename VT, bool PAIR>
 __global__ void __launch_bounds__(128) sddmm_dmma_kernel(int n_block_rows, int n_chunks, int b,
@@ -135,12 +137,12 @@ __global__ void __launch_bounds__(128) sddmm_dmma_kernel(int n_block_rows, int n
             const int n = min(col0 + 8 * u + fr, cols - 1), blk = n / b;
             Tr[u] = T + (int64_t(__ldg(col_ind + kb + blk)) * b + (n - blk * b)) * R;
         }
-        // Two sums a tile, of the even and the odd k': half the chain each (its
-        // length shows in the rounding).
-        double acc[2][kSdTiles][2];
+        // Sums of kSdFold steps, and of those (one chain of all terms shows its
+        // length in the rounding).
+        double acc[kSdTiles][2], sum[kSdTiles][2];
 #pragma unroll
         for (int u = 0; u < kSdTiles; ++u)
-            acc[0][u][0] = acc[0][u][1] = acc[1][u][0] = acc[1][u][1] = 0.0;
+            acc[u][0] = acc[u][1] = sum[u][0] = sum[u][1] = 0.0;
         // (q, s) of this lane's two k'
         int q0 = 2 * fc / R, s0 = 2 * fc - q0 * R;
         int q1 = (2 * fc + 1) / R, s1 = 2 * fc + 1 - q1 * R;
@@ -169,8 +171,17 @@ __global__ void __launch_bounds__(128) sddmm_dmma_kernel(int n_block_rows, int n
             const double a1 = v1 ? (n0 + q1 ? 2.0 : 1.0) * double(l1) : 0.0;
 #pragma unroll
             for (int u = 0; u < kSdTiles; ++u) {
-                dmma_884(acc[0][u], a0, v0 ? double(t0[u]) : 0.0);
-                dmma_884(acc[1][u], a1, v1 ? double(t1[u]) : 0.0);
+                dmma_884(acc[u], a0, v0 ? double(t0[u]) : 0.0);
+                dmma_884(acc[u], a1, v1 ? double(t1[u]) : 0.0);
+            }
+            if ((t >> 3) % kSdFold == kSdFold - 1) {  // one step for all lanes: t / 8
+#pragma unroll
+                for (int u = 0; u < kSdTiles; ++u)
+#pragma unroll
+                    for (int v = 0; v < 2; ++v) {
+                        sum[u][v] += acc[u][v];
+                        acc[u][v] = 0.0;
+                    }
             }
             q0 += dq;
             s0 += ds;
@@ -193,7 +204,7 @@ __global__ void __launch_bounds__(128) sddmm_dmma_kernel(int n_block_rows, int n
                     const int n = col0 + 8 * u + 2 * fc + v, blk = n / b;
                     if (n < cols)
                         grad[(int64_t(kb + blk) * b + fr) * b + (n - blk * b)] +=
-                            scale * (acc[0][u][v] + acc[1][u][v]);
+                            scale * (sum[u][v] + acc[u][v]);
                 }
         }
     }
